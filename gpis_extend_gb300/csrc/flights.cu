@@ -8,9 +8,9 @@
 //              (SparseConvolutionNoiseMedium.cpp:287-346): persistent warps pull
 //              flights from a device work counter and refill finished lanes, so
 //              flights of very uneven length keep every lane busy; value-only
-//              field evaluations; the 1D variant keeps the impulses of the three
-//              cells around the query in registers and regenerates a cell only
-//              when the query crosses a cell boundary;
+//              field evaluations; the impulses of the cells around the query are kept
+//              and a cell is generated only when the query comes near it; 3D media give
+//              a flight to a group of lanes that share its impulses;
 //   k_finish   the gradient sample at the end point (evaluateGradient,
 //              SparseConvolutionNoise.cpp:133-296), one thread per flight.
 //
@@ -1838,6 +1838,7 @@ __device__ float field_precise(const LaneField &L, float px, float py, float pz,
 // Generic evaluator: recomputes every impulse (any impulse count, 1D or 3D).
 struct EvalGeneric {
     static constexpr bool kCollective = false;
+    static constexpr int kGroup = 1;
     static constexpr int kMinBlocks = 2;
     static constexpr bool kGeneral = true;
     static constexpr bool kSkip = false;
@@ -1984,6 +1985,56 @@ __device__ __forceinline__ bool cert_fac(float pf, float fb, float eps, float &d
     return isfinite(dfac);
 }
 
+// The conditioning splat's range along the segment [p, p + len d], added to [nlo, nhi].
+__device__ __forceinline__ void cond3d_range(const DevMedium &m, const LaneField &L, const float p[3], const float d[3],
+                                             float len, float &nlo, float &nhi)
+{
+    // exponent -log2e Q(s), Q(s) = C + 2 B s + A s^2 over s in [0, 1]
+    float A = 0.0f, B = 0.0f, C = 0.0f, gh = 0.0f, eh = 0.0f;
+    const CondOct &co = L.c3.oct[0];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        const float ab = p[i] - L.o[i], ew = len * d[i];
+        A += m.m3c[i] * ew * ew;
+        B += m.m3c[i] * ab * ew;
+        C += m.m3c[i] * ab * ab;
+        gh += ab * m.m3c[i] * co.gs[i];
+        eh += ew * m.m3c[i] * co.gs[i];
+    }
+    const float sn = A > 0.0f ? fminf(fmaxf(-B / A, 0.0f), 1.0f) : 0.0f;
+    const float qmin = fmaxf(C + sn * (2.0f * B + sn * A), 0.0f);
+    const float qmax = fmaxf(C, C + 2.0f * B + A);
+    const float fmax = ex2_approx(-LOG2E * qmin) * 1.00001f;
+    const float fmin = ex2_approx(-LOG2E * qmax) * 0.99999f;
+    const float vlo = co.vs >= 0.0f ? co.vs * fmin : co.vs * fmax;
+    const float vhi = co.vs >= 0.0f ? co.vs * fmax : co.vs * fmin;
+    const float gb = 2.0f * fmax * (fabsf(gh) + fabsf(eh)) * 1.00001f;
+    nlo += vlo - gb;
+    nhi += vhi + gb;
+}
+
+// The field's range over the segment from the noise's and the mean mu at its start.
+__device__ __forceinline__ void field_range_3d(const DevMedium &m, const LaneField &L, const float d[3], float len,
+                                               float mu, float nlo, float nhi, float &f_lo, float &f_hi)
+{
+    const float dn = sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
+    const float dm = m.skip_mean_lip * len * dn * 1.0001f;
+    const float sg = L.sigma;
+    f_lo = (sg >= 0.0f ? sg * nlo : sg * nhi) + mu - dm;
+    f_hi = (sg >= 0.0f ? sg * nhi : sg * nlo) + mu + dm;
+}
+
+// Steps of length `step` after a point of value f that keep its sign, from the range
+// [f_lo, f_hi] over the next dlen.
+__device__ __forceinline__ int range_skips(float dlen, float f_lo, float f_hi, float f, float step, int cap)
+{
+    if (!(dlen > 0.0f)) return 0;
+    const float margin = 1e-5f + 1e-6f * fmaxf(fabsf(f_lo), fabsf(f_hi));
+    const bool keep = f > 0.0f ? f_lo > margin : (f < 0.0f && f_hi < -margin);
+    if (!keep) return 0;
+    return (int)fminf(floorf(dlen / step * (1.0f - 1e-6f)), (float)cap);
+}
+
 // 3D stationary single-octave media with step skipping.  The value is EvalGeneric's
 // (the same arithmetic); a march step that plans a segment [p, p + D d] also gets the
 // range of the field over it: the raw noise sum's range (noise3d_core), the
@@ -1996,6 +2047,7 @@ __device__ __forceinline__ bool cert_fac(float pf, float fb, float eps, float &d
 // reference would march past: those steps are skipped.
 struct EvalSkip3D {
     static constexpr bool kCollective = false;
+    static constexpr int kGroup = 1;
     static constexpr int kMinBlocks = 2;
     static constexpr bool kGeneral = true;
     static constexpr bool kSkip = false;
@@ -2051,51 +2103,351 @@ struct EvalSkip3D {
             float cv, cg[3];
             cond3d(m, L.c3, L.o, p, cv, cg);
             noise += cv;
-            if (len > 0.0f) {
-                // exponent -log2e Q(s), Q(s) = C + 2 B s + A s^2 over s in [0, 1]
-                float A = 0.0f, B = 0.0f, C = 0.0f, gh = 0.0f, eh = 0.0f;
-                const CondOct &co = L.c3.oct[0];
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    const float ab = p[i] - L.o[i], ew = len * d[i];
-                    A += m.m3c[i] * ew * ew;
-                    B += m.m3c[i] * ab * ew;
-                    C += m.m3c[i] * ab * ab;
-                    gh += ab * m.m3c[i] * co.gs[i];
-                    eh += ew * m.m3c[i] * co.gs[i];
-                }
-                const float sn = A > 0.0f ? fminf(fmaxf(-B / A, 0.0f), 1.0f) : 0.0f;
-                const float qmin = fmaxf(C + sn * (2.0f * B + sn * A), 0.0f);
-                const float qmax = fmaxf(C, C + 2.0f * B + A);
-                const float fmax = ex2_approx(-LOG2E * qmin) * 1.00001f;
-                const float fmin = ex2_approx(-LOG2E * qmax) * 0.99999f;
-                const float vlo = co.vs >= 0.0f ? co.vs * fmin : co.vs * fmax;
-                const float vhi = co.vs >= 0.0f ? co.vs * fmax : co.vs * fmin;
-                const float gb = 2.0f * fmax * (fabsf(gh) + fabsf(eh)) * 1.00001f;
-                nlo += vlo - gb;
-                nhi += vhi + gb;
-            }
+            if (len > 0.0f) cond3d_range(m, L, p, d, len, nlo, nhi);
         }
         const float mu = lane_mean(L, px, py, pz, id);
         if (len > 0.0f) {
-            const float dn = sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-            const float dm = m.skip_mean_lip * len * dn * 1.0001f;
-            const float sg = L.sigma;
-            f_lo = (sg >= 0.0f ? sg * nlo : sg * nhi) + mu - dm;
-            f_hi = (sg >= 0.0f ? sg * nhi : sg * nlo) + mu + dm;
+            field_range_3d(m, L, d, len, mu, nlo, nhi, f_lo, f_hi);
             dlen = len;
         }
         return L.sigma * noise + mu;
     }
 
-    // steps of length `step` after p that keep the sign of f (f the value at p)
     __device__ __forceinline__ int skips(float f, float step, int cap) const
     {
-        if (!(dlen > 0.0f)) return 0;
-        const float margin = 1e-5f + 1e-6f * fmaxf(fabsf(f_lo), fabsf(f_hi));
-        const bool keep = f > 0.0f ? f_lo > margin : (f < 0.0f && f_hi < -margin);
-        if (!keep) return 0;
-        return (int)fminf(floorf(dlen / step * (1.0f - 1e-6f)), (float)cap);
+        return range_skips(dlen, f_lo, f_hi, f, step, cap);
+    }
+};
+
+// Lane groups.  An evaluator with kGroup = G > 1 gives a flight to G neighbouring
+// lanes, which run the march's state machine on the same values and share the
+// impulses: every branch is taken by the whole group, and only the group's first
+// lane writes.
+__device__ __forceinline__ unsigned group_mask(int g)
+{
+    return g == 32 ? FULL : (((1u << (g & 31)) - 1u) << ((threadIdx.x & 31) & ~(g - 1)));
+}
+
+template <int G>
+__device__ __forceinline__ float group_sum(float v, unsigned mask)
+{
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) v += __shfl_xor_sync(mask, v, o);
+    return v;
+}
+
+// 3D stationary single-octave media with at most 8 impulses per cell: G lanes per
+// flight, lane k % 8 of each eight carrying impulse k of every cell.  The 27 cells
+// around the query sit in shared memory, in the slot given by their coordinates
+// modulo 3 (counted from where the block was first filled), so that moving to a
+// neighbouring cell generates the 9 cells that come into
+// the block and leaves the others where they are.  A lane's evaluation is then one
+// 16-byte load and about 20 instructions per impulse, where EvalSkip3D draws all 216
+// impulses again (about 70 instructions each).  Values and ranges are EvalSkip3D's up
+// to the order of the sums; precise() repeats noise3d_precise, whose sums run over the
+// impulses of a cell and then over the cells in order.  What bounds it: issue slots (65 %
+// busy at 40 009 flights, the range's 27 x 39 instructions per lane first, then the
+// cells that come in), 2 CTAs per SM by registers and by the blocks' 108 KB.  Fast pass
+// and resume pass of 40 009 sphere-field flights: 7.0 and 1.9 ms with EvalSkip3D and
+// EvalGeneric, 0.95 and 0.35 ms here; the 96 x 96, 4 spp image with 3D noise 52.7 -> 5.5 ms.
+constexpr int kG3Threads = 256;
+constexpr int kG3Imp = 8;
+// Batches below this size take a warp per flight, larger ones eight lanes.  The warp
+// finishes a flight sooner (256 flights: 0.32 against 0.45 ms a batch, 5 000: 0.53 / 0.59),
+// the eight lanes repeat less work per flight (10 000: 0.760 / 0.755, 40 009: 1.86 / 1.47).
+constexpr uint32_t kG3Few = 10000;
+template <int G>
+constexpr size_t kSmemG3 = (size_t)(kG3Threads / G) * 27 * kG3Imp * sizeof(float4);
+
+template <int G>
+struct EvalGroup3D {
+    static constexpr bool kCollective = false;
+    static constexpr int kGroup = G;
+    static constexpr int kMinBlocks = 2;
+    static constexpr bool kGeneral = true;
+    static constexpr bool kSkip = false;
+    static_assert(G == 8 || G == 32, "eight lanes per cell: one cell at a time, or a row of three");
+    float want, dlen, f_lo, f_hi;           // as EvalSkip3D
+    int cx, cy, cz;                         // the cell the block is centred on
+    int rx, ry, rz;                         // its coordinates modulo 3
+    bool valid;
+    float4 *cells;                          // the group's 27 x 8 impulses: position, weight
+    const PcgJump *sj;
+    unsigned mask;
+
+    __device__ __forceinline__ void reset() { want = 0.0f; dlen = 0.0f; valid = false; cx = cy = cz = rx = ry = rz = 0; }
+    __device__ __forceinline__ void bind(const PcgJump *t)
+    {
+        extern __shared__ float4 dsm_g3[];
+        cells = dsm_g3 + (threadIdx.x / G) * (27 * kG3Imp);
+        sj = t;
+        mask = group_mask(G);
+    }
+    __device__ __forceinline__ void plan(float len) { want = len; }
+
+    // the residue of the neighbour at offset o (-1, 0, 1) of one whose residue is r
+    static __device__ __forceinline__ int wrap3(int r, int o)
+    {
+        r += o;
+        return r < 0 ? 2 : (r > 2 ? 0 : r);
+    }
+
+    // the impulses of `count` cells: cell(j) gives the offset of the j-th from the centre.
+    // Each lane of eight hashes one cell for the eight, then draws impulse k of each.
+    template <class Cell>
+    __device__ __forceinline__ void draw(int count, const DevMedium &m, uint32_t seed, Cell cell)
+    {
+        const int k = threadIdx.x & 7, j0 = (threadIdx.x & (G - 1)) >> 3;
+        const bool xfirst = (m.flags & MF_XYZ_ORDER) != 0;
+        constexpr int kSub = G / 8;     // cells side by side
+#pragma unroll 1
+        for (int base = 0; base < count; base += G) {
+            int x, y, z;
+            cell(base + k * kSub + j0, x, y, z);
+            const uint32_t h = xxhash4((uint32_t)cz + (uint32_t)z, (uint32_t)cy + (uint32_t)y,
+                                       (uint32_t)cx + (uint32_t)x, seed) + 1u;
+            const int slot = (wrap3(rx, x) * 9 + wrap3(ry, y) * 3 + wrap3(rz, z)) * kG3Imp;
+#pragma unroll 1
+            for (int i = 0; i < 8 && base + i * kSub < count; ++i) {
+                const uint32_t s = __shfl_sync(mask, h, i, 8);
+                const int to = __shfl_sync(mask, slot, i, 8) + k;
+                if (kSub > 1 && base + i * kSub + j0 >= count) continue;
+                float4 q = make_float4(4.0f, 4.0f, 4.0f, 0.0f);     // out of every query's reach
+                if ((uint32_t)k < m.n_imp) {
+                    const int b = 2 + 4 * k;
+                    const float r0 = unit_float(pcg_draw(sj[b], s));
+                    const float r1 = unit_float(pcg_draw(sj[b + 1], s));
+                    const float r2 = unit_float(pcg_draw(sj[b + 2], s));
+                    const uint32_t wr = pcg_draw(sj[b + 3], s);
+                    q = make_float4(xfirst ? r0 : r2, r1, xfirst ? r2 : r0, (wr >> 31) ? 1.0f : -1.0f);
+                }
+                cells[to] = q;
+            }
+        }
+    }
+
+    // the block of 27 cells around (x, y, z)
+    __device__ __forceinline__ void move(int x, int y, int z, const DevMedium &m, uint32_t seed)
+    {
+        if (valid && x == cx && y == cy && z == cz) return;
+        // one step along one axis (within the range where x + 1 does not wrap): the
+        // centre's residues follow, and the face that comes in is drawn
+        const int ux = x - cx, uy = y - cy, uz = z - cz;
+        const bool near_by = valid && abs(ux) + abs(uy) + abs(uz) == 1 && max(max(abs(x), abs(y)), abs(z)) < (1 << 30);
+        if (near_by) {
+            rx = wrap3(rx, ux);
+            ry = wrap3(ry, uy);
+            rz = wrap3(rz, uz);
+        } else {
+            rx = ry = rz = 1;
+        }
+        cx = x;
+        cy = y;
+        cz = z;
+        valid = true;
+        __syncwarp(mask);       // every lane has read the old block
+        draw(near_by ? 9 : 27, m, seed, [&](int j, int &ox, int &oy, int &oz) {
+            const int a = j / 9, b = (j / 3) % 3 - 1, c = j % 3 - 1;
+            ox = near_by ? (ux ? ux : b) : min(a, 2) - 1;
+            oy = near_by ? (uy ? uy : (ux ? b : c)) : b;
+            oz = near_by && uz ? uz : c;
+        });
+        __syncwarp(mask);
+    }
+
+    struct Query {
+        float t[3][3];          // fraction minus the cell offset, per axis
+        int sx[3], sy[3], sz[3];  // slot of each offset
+    };
+    __device__ __forceinline__ void locate(const LaneField &L, const float p[3], Query &q)
+    {
+        const DevMedium &m = *L.m;
+        int c[3];
+#pragma unroll
+        for (int i = 0; i < 3; ++i) {
+            const float v = __fdiv_rn(p[i], m.kr_world);
+            const float fl = floorf(v);
+            const float fr = __fsub_rn(v, fl);
+            c[i] = (int)fl;
+#pragma unroll
+            for (int o = 0; o < 3; ++o) q.t[i][o] = __fsub_rn(fr, (float)(o - 1));
+        }
+        move(c[0], c[1], c[2], m, L.seed);
+#pragma unroll
+        for (int o = 0; o < 3; ++o) {
+            q.sx[o] = wrap3(rx, o - 1) * 9;
+            q.sy[o] = wrap3(ry, o - 1) * 3;
+            q.sz[o] = wrap3(rz, o - 1);
+        }
+    }
+    static __device__ __forceinline__ float pick(const float t[3], int o) { return o == 0 ? t[0] : (o == 1 ? t[1] : t[2]); }
+    static __device__ __forceinline__ int pick(const int t[3], int o) { return o == 0 ? t[0] : (o == 1 ? t[1] : t[2]); }
+
+    template <bool BOUND>
+    __device__ __forceinline__ void sums(const DevMedium &m, const Query &q, const float E[3], float ee, float kmax2,
+                                         float kmin2, float &sv, float &lo, float &hi) const
+    {
+        const float kr = m.kr_world;
+        const float k0 = m.kexp3d[0] * kr * kr, k1 = m.kexp3d[1] * kr * kr, k2 = m.kexp3d[2] * kr * kr;
+        const float iee = ee > 0.0f ? -1.0f / ee : 0.0f;
+        const int k = threadIdx.x & 7;
+        sv = lo = hi = 0.0f;
+        auto one = [&](float t0, float t1, float t2, int slot) {
+            const float4 c = cells[slot * kG3Imp + k];
+            const float a0 = __fsub_rn(t0, c.x), a1 = __fsub_rn(t1, c.y), a2 = __fsub_rn(t2, c.z);
+            const float s0 = __fmul_rn(a0, a0), s1 = __fmul_rn(a1, a1), s2 = __fmul_rn(a2, a2);
+            const float l2 = __fadd_rn(__fadd_rn(s0, s1), s2);
+            const float e = ex2_approx(k0 * s0 + (k1 * s1 + k2 * s2));
+            sv += l2 < 1.0f ? c.w * e : 0.0f;
+            if (BOUND) {
+                // 1.4427e-5 = log2(1 + 1e-5): the outward margin against ex2.approx
+                const float ae = a0 * E[0] + a1 * E[1] + a2 * E[2];
+                const float ae2 = 2.0f * ae;
+                const float sn = __saturatef(ae * iee);
+                const float b2 = l2 + sn * (ae2 + sn * ee);
+                const float far2 = fmaxf(l2, (l2 + ae2) + ee);
+                const float big = b2 < 1.0f + kSupportEps ? c.w * ex2_approx(kmax2 * b2 + 1.4427e-5f) : 0.0f;
+                const float small = far2 < 1.0f - kSupportEps ? c.w * ex2_approx(kmin2 * far2 - 1.4427e-5f) : 0.0f;
+                lo += fminf(big, small);
+                hi += fmaxf(big, small);
+            }
+        };
+        if constexpr (G == 8) {
+#pragma unroll 1
+            for (int x = 0; x < 3; ++x) {
+                const float t0 = pick(q.t[0], x);
+                const int sx = pick(q.sx, x);
+#pragma unroll
+                for (int y = 0; y < 3; ++y)
+#pragma unroll
+                    for (int z = 0; z < 3; ++z) one(t0, q.t[1][y], q.t[2][z], sx + q.sy[y] + q.sz[z]);
+            }
+        } else {
+            // a warp: eight lanes for each of a row's three cells, the last eight idle
+            const int z = min((int)(threadIdx.x & 31) >> 3, 2);
+            const float t2 = (threadIdx.x & 24) == 24 ? 8.0f : pick(q.t[2], z);
+            const int sz = pick(q.sz, z);
+#pragma unroll
+            for (int x = 0; x < 3; ++x)
+#pragma unroll
+                for (int y = 0; y < 3; ++y) one(q.t[0][x], q.t[1][y], t2, q.sx[x] + q.sy[y] + sz);
+        }
+        sv = group_sum<G>(sv, mask);
+        if (BOUND) {
+            lo = group_sum<G>(lo, mask);
+            hi = group_sum<G>(hi, mask);
+        }
+    }
+
+    __device__ __forceinline__ float value(const LaneField &L, const float d[3], float px, float py, float pz, int &id,
+                                           uint32_t &refills, bool)
+    {
+        const DevMedium &m = *L.m;
+        refills += 27;
+        const float p[3] = {px, py, pz};
+        float len = want;
+        want = 0.0f;
+        dlen = 0.0f;
+        const float kr = m.kr_world;
+        Query q;
+        locate(L, p, q);
+        // the segment's end inside p's cell (EvalSkip3D)
+        if (len > 0.0f && m.skip_mean_lip >= 0.0f) {
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+                const float fr = q.t[i][1];
+                const float di = d[i] / kr;
+                float room = 1e30f;
+                if (di > 0.0f) room = (1.0f - kSupportEps - fr) / di;
+                else if (di < 0.0f) room = (fr - kSupportEps) / -di;
+                len = fminf(len, room);
+            }
+        } else {
+            len = 0.0f;
+        }
+        float v, lo = 0.0f, hi = 0.0f;
+        const float E[3] = {len * d[0] / kr, len * d[1] / kr, len * d[2] / kr};
+        const float ee = E[0] * E[0] + E[1] * E[1] + E[2] * E[2];
+        const bool bound = len > 0.0f && ee > 0.0f;
+        // one of the groups of this warp wants a range: all of them run that form, which
+        // costs less than both forms one after the other
+        if (__any_sync(__activemask(), bound)) {
+            const float kr2 = kr * kr;
+            const float kmax2 = fmaxf(fmaxf(m.kexp3d[0], m.kexp3d[1]), m.kexp3d[2]) * kr2;
+            const float kmin2 = fminf(fminf(m.kexp3d[0], m.kexp3d[1]), m.kexp3d[2]) * kr2;
+            sums<true>(m, q, E, ee, kmax2, kmin2, v, lo, hi);
+        } else {
+            sums<false>(m, q, E, 0.0f, 0.0f, 0.0f, v, lo, hi);
+        }
+        float noise = v * m.inv_norm3d;
+        float nlo = lo * m.inv_norm3d, nhi = hi * m.inv_norm3d;
+        if (L.cond) {
+            float cv, cg[3];
+            cond3d(m, L.c3, L.o, p, cv, cg);
+            noise += cv;
+            if (bound) cond3d_range(m, L, p, d, len, nlo, nhi);
+        }
+        const float mu = lane_mean(L, px, py, pz, id);
+        if (bound) {
+            field_range_3d(m, L, d, len, mu, nlo, nhi, f_lo, f_hi);
+            dlen = len;
+        }
+        return L.sigma * noise + mu;
+    }
+
+    __device__ __forceinline__ int skips(float f, float step, int cap) const
+    {
+        return range_skips(dlen, f_lo, f_hi, f, step, cap);
+    }
+
+    __device__ __forceinline__ float precise(const LaneField &L, const float p[3], int &id)
+    {
+        const DevMedium &m = *L.m;
+        const float kr = m.kr_world;
+        const int k = threadIdx.x & 7;
+        Query q;
+        locate(L, p, q);
+        float sv = 0.0f;
+        // a cell's impulse as noise3d_precise evaluates it; one that is out of reach adds
+        // +0, which leaves a sum that started at +0 as it is
+        auto one = [&](float t0, float t1, float t2, int slot) {
+            const float4 c = cells[slot * kG3Imp + k];
+            const float a0 = __fsub_rn(t0, c.x), a1 = __fsub_rn(t1, c.y), a2 = __fsub_rn(t2, c.z);
+            const float l2 = __fadd_rn(__fadd_rn(__fmul_rn(a0, a0), __fmul_rn(a1, a1)), __fmul_rn(a2, a2));
+            float e = 0.0f;
+            if (l2 < 1.0f) {
+                const float b0 = __fsub_rn(__fmul_rn(kr, t0), __fmul_rn(kr, c.x));
+                const float b1 = __fsub_rn(__fmul_rn(kr, t1), __fmul_rn(kr, c.y));
+                const float b2 = __fsub_rn(__fmul_rn(kr, t2), __fmul_rn(kr, c.z));
+                float w = __fmul_rn(__fmul_rn(b0, m.m3[0]), b0);
+                w = __fadd_rn(w, __fmul_rn(__fmul_rn(b1, m.m3[1]), b1));
+                w = __fadd_rn(w, __fmul_rn(__fmul_rn(b2, m.m3[2]), b2));
+                e = cr_expf(-w);
+                if (c.w < 0.0f) e = -e;
+            }
+            // the cell's sum in impulse order
+            float cv = 0.0f;
+#pragma unroll
+            for (int i = 0; i < kG3Imp; ++i) cv = __fadd_rn(cv, __shfl_sync(mask, e, i, 8));
+            return cv;
+        };
+        const int z0 = min((int)(threadIdx.x & (G - 1)) >> 3, 2);
+#pragma unroll 1
+        for (int j = 0; j < 9; ++j) {
+            const float t0 = pick(q.t[0], j / 3), t1 = pick(q.t[1], j % 3);
+            const int slot = pick(q.sx, j / 3) + pick(q.sy, j % 3);
+            if constexpr (G == 8) {
+#pragma unroll 1
+                for (int z = 0; z < 3; ++z) sv = __fadd_rn(sv, one(t0, t1, pick(q.t[2], z), slot + pick(q.sz, z)));
+            } else {
+                const float cv = one(t0, t1, pick(q.t[2], z0), slot + pick(q.sz, z0));
+#pragma unroll
+                for (int z = 0; z < 3; ++z) sv = __fadd_rn(sv, __shfl_sync(mask, cv, 8 * z));
+            }
+        }
+        float noise = __fdiv_rn(sv, m.norm3d);
+        if (L.cond) noise = __fadd_rn(noise, cond3d_value_precise(m, L.c3, L.o, p));
+        return mean_plus_precise(m, __fmul_rn(L.sigma, noise), p[0], p[1], p[2], id);
     }
 };
 
@@ -2115,6 +2467,7 @@ constexpr size_t kSmem1D = (size_t)3 * 8 * sizeof(float) * kC1Threads;
 template <int NMAX, bool GRID = false, bool NS = false, bool SM = false>
 struct EvalCoop1D {
     static constexpr bool kCollective = true;
+    static constexpr int kGroup = 1;
     // CTAs per SM for the stationary analytic-mean kernel: with the window in shared
     // memory 3 (80 registers; 14.34 ms per bench step against 14.72 for 4 CTAs at 64
     // registers, whose spills feed long-scoreboard stalls, and 15.44 for 2 at 128),
@@ -2341,6 +2694,7 @@ constexpr size_t kSmemOct = (size_t)kOctMax * 3 * 8 * sizeof(float) * kOctThread
 
 struct EvalCoopOct {
     static constexpr bool kCollective = true;
+    static constexpr int kGroup = 1;
     static constexpr int kMinBlocks = 2;
     static constexpr bool kGeneral = true;
     static constexpr bool kSkip = false;
@@ -2586,6 +2940,7 @@ template <> struct IsOct<EvalCoop1D<8, false, true>> { static constexpr bool val
 
 template <class E> struct IsSkip3D { static constexpr bool value = false; };
 template <> struct IsSkip3D<EvalSkip3D> { static constexpr bool value = true; };
+template <int G> struct IsSkip3D<EvalGroup3D<G>> { static constexpr bool value = true; };
 
 template <class Eval>
 __device__ __forceinline__ float eval_at(Eval &ev, const LaneField &L, const float *, const float p[3], int &id,
@@ -2594,6 +2949,12 @@ __device__ __forceinline__ float eval_at(Eval &ev, const LaneField &L, const flo
     return ev.value(L, p[0], p[1], p[2], id, refills, live);
 }
 __device__ __forceinline__ float eval_at(EvalSkip3D &ev, const LaneField &L, const float *d, const float p[3],
+                                         int &id, uint32_t &refills, bool live)
+{
+    return ev.value(L, d, p[0], p[1], p[2], id, refills, live);
+}
+template <int G>
+__device__ __forceinline__ float eval_at(EvalGroup3D<G> &ev, const LaneField &L, const float *d, const float p[3],
                                          int &id, uint32_t &refills, bool live)
 {
     return ev.value(L, d, p[0], p[1], p[2], id, refills, live);
@@ -2685,17 +3046,23 @@ __device__ __forceinline__ unsigned long long warp_sum(uint32_t v)
 // where that is certain and hands the rest on (kResumeNoCert) to the precise pass,
 // so that no warp runs both evaluators.
 template <class Eval, bool RESUME, bool CERT = false>
-__global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
+__device__ __forceinline__ void march_flights(const FlightArgs &a)
 {
     static_assert(!CERT || RESUME, "the certified pass is a resume pass");
     const int lane = threadIdx.x & 31;
+    // the first lane of the flight's group fetches, writes and counts for it
+    constexpr int G = Eval::kGroup;
+    const bool lead = G == 1 || (lane & (G - 1)) == 0;
+    const uint32_t one = lead ? 1u : 0u;
+    constexpr bool kOwn3D = G > 1 && IsSkip3D<Eval>::value;     // marches on with its own evaluator
     uint32_t *work = a.work + (RESUME ? (CERT ? 1 : 2) : 0);
-    const unsigned lt_mask = (1u << lane) - 1u;
+    const unsigned lt_mask = (1u << (lane & ~(G - 1))) - 1u;
     // 0.9 and 0.01 as float-float pairs (the reference's double constants)
     const FF kNine = {0.9f, -2.38418579e-08f};
     const float kHundredthH = 0.01f, kHundredthL = -2.23517418e-10f;
-    __shared__ PcgJump s_jump[2 + 2 * 8];
-    if (threadIdx.x < 2 + 2 * 8) s_jump[threadIdx.x] = c_jump[threadIdx.x];
+    constexpr int kJumps = 2 + (kOwn3D ? 4 : 2) * 8;
+    __shared__ PcgJump s_jump[kJumps];
+    if (threadIdx.x < kJumps) s_jump[threadIdx.x] = c_jump[threadIdx.x];
     __syncthreads();
     Eval ev;
     ev.reset();
@@ -2731,7 +3098,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
 
     for (;;) {
         const bool need = phase == PH_IDLE && !drained;
-        const unsigned need_mask = __ballot_sync(FULL, need);
+        const unsigned need_mask = __ballot_sync(FULL, need && lead);
         if (need_mask) {
             const int leader = __ffs(need_mask) - 1;
             uint32_t base = 0;
@@ -2744,7 +3111,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                 } else {
                     const uint32_t idx = q_in ? queue_in[item] : item;
                     fid = idx;
-                    if (!RESUME) c_flights++;
+                    if (!RESUME) c_flights += one;
                     prop_a = (!RESUME && a.proposal) ? a.proposal[idx].x : -INFINITY;
                     bool mok;
                     L.m = medium_of(a, idx, mok);
@@ -2756,7 +3123,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                     } else if (CERT && ((rs.w >> 28) != (uint32_t)PH_MARCH_P || (rs.w & kResumeNoCert) || !mok ||
                                         !cert_medium(m))) {
                         // left to the precise pass
-                        if (queue_out) queue_push(queue_out, queue_len, idx);
+                        if (queue_out && lead) queue_push(queue_out, queue_len, idx);
                     } else if (Eval::kSkip && !RESUME && a.setup) {
                         // the set-up k_prepare computed for this flight
                         const float4 s0 = a.setup[4 * (size_t)idx], s1 = a.setup[4 * (size_t)idx + 1];
@@ -2764,10 +3131,12 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                         const uint32_t flags = __float_as_uint(s3.y);
                         const float4 on = a.origin_near[idx], df = a.dir_far[idx];
                         if (!mok || !(flags & SF_VALID)) {
-                            write_status(a, idx, 0.0f, 0.0f, 1.0f, 0u, GPIS_FLIGHT_INVALID_INPUT);
-                            a.t_end[idx] = 0.0;
-                            a.resume[idx] = make_uint4(0u, 0u, 0u, 0u);
-                            c_invalid++;
+                            if (lead) {
+                                write_status(a, idx, 0.0f, 0.0f, 1.0f, 0u, GPIS_FLIGHT_INVALID_INPUT);
+                                a.t_end[idx] = 0.0;
+                                a.resume[idx] = make_uint4(0u, 0u, 0u, 0u);
+                            }
+                            c_invalid += one;
                         } else {
 #pragma unroll
                             for (int k = 0; k < 3; ++k) L.li[k] = m.l_inv[k];
@@ -2806,10 +3175,12 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                             phase = PH_F0;
                         }
                     } else if (const FlightIn fl = load_flight(a, idx); !mok || !flight_valid(fl)) {
-                        write_status(a, idx, 0.0f, 0.0f, 1.0f, 0u, GPIS_FLIGHT_INVALID_INPUT);
-                        a.t_end[idx] = 0.0;
-                        a.resume[idx] = make_uint4(0u, 0u, 0u, 0u);
-                        c_invalid++;
+                        if (lead) {
+                            write_status(a, idx, 0.0f, 0.0f, 1.0f, 0u, GPIS_FLIGHT_INVALID_INPUT);
+                            a.t_end[idx] = 0.0;
+                            a.resume[idx] = make_uint4(0u, 0u, 0u, 0u);
+                        }
+                        c_invalid += one;
                     } else {
 #pragma unroll
                         for (int k = 0; k < 3; ++k) d[k] = fl.d[k];
@@ -2868,13 +3239,13 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
         if constexpr (IsSkip3D<Eval>::value) {
             // a marching step of a 3D medium asks for the field's range over the next
             // steps: about half of |f| at the last step, and at least two steps
-            if (!RESUME && phase == PH_MARCH) {
+            if ((!RESUME || kOwn3D) && phase == PH_MARCH) {
                 const float len = fminf(0.5f * fabsf(pf), (float)kMaxSkip3D * step);
                 ev.plan(len >= 2.0f * step ? len : 0.0f);
             }
         }
         bool use3 = false;
-        if constexpr (RESUME) {
+        if constexpr (RESUME && !kOwn3D) {
             const DevMedium &m3 = *L.m;
             use3 = !precise && phase == PH_MARCH && !(m3.flags & MF_ONE_D) && m3.n_oct == 1 && !general_3d(m3);
             if (use3) {
@@ -2889,6 +3260,9 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
             f = value_1d_cert(L, p[0], p[1], p[2], id, margin);
             c_refills += 3;
         } else {
+            if constexpr (kOwn3D) {
+                f = precise ? ev.precise(L, p, id) : eval_at(ev, L, d, p, id, c_refills, live);
+            } else
             f = precise ? field_precise(L, p[0], p[1], p[2], id)
                         : (use3 ? ev3.value(L, d, p[0], p[1], p[2], id, c_refills, live)
                                 : eval_at(ev, L, d, p, id, c_refills, live));
@@ -2924,7 +3298,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
             // (t stays at tb through the refinement)
             if (phase != PH_MARCH_P) {
                 steps--;
-                c_steps--;
+                c_steps -= one;
                 pf_precise = false;
                 phase = PH_MARCH_P;
             }
@@ -2933,7 +3307,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
             // a non-finite field value ends the flight (RaySegmentBatch.cu:228-229, 238-239)
             done = true;
             status = GPIS_FLIGHT_INVALID_INPUT;
-            c_invalid++;
+            c_invalid += one;
         } else if (phase == PH_F0 && first && fabsf(f) < kPreciseBand) {
             // the initial sign decides the crossing of a primary flight; a secondary
             // flight takes its sign from the first step instead
@@ -2958,7 +3332,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
             pend = !RESUME || CERT;
         } else if (phase == PH_MARCH || phase == PH_MARCH_P) {
             steps++;
-            c_steps++;
+            c_steps += one;
             bool crossed = false;
             if (!first && steps == 1) {
                 sign0 = sg;
@@ -2986,7 +3360,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                     if (CERT && !cert_fac(pf, fb, kPreciseBand, dfac)) {
                         // too close to call: the precise pass, from tb
                         steps--;
-                        c_steps--;
+                        c_steps -= one;
                         pf_precise = false;
                         phase = PH_MARCH_P;
                         pend = true;
@@ -3012,7 +3386,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                     if (af > per) skip = (int)fminf(af / per, cap);
                 }
                 if constexpr (IsSkip3D<Eval>::value) {
-                    if (!RESUME) skip = ev.skips(f, step, kMaxSkip3D);
+                    if (!RESUME || kOwn3D) skip = ev.skips(f, step, kMaxSkip3D);
                 }
                 if constexpr (IsOct<Eval>::value) {
                     if (!RESUME)
@@ -3024,7 +3398,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                     // (1D media) or range bound (3D media); the value before a later
                     // crossing is then no longer the last one evaluated, so the refinement
                     // re-evaluates it
-                    if (L.m->flags & MF_ONE_D)
+                    if (!kOwn3D && (L.m->flags & MF_ONE_D))
                         skip = oct_skip_count(*L.m, L, d, ns_scale(*L.m, p[0], p[2]), f, step, kMaxSkip);
                     else if (use3)
                         skip = ev3.skips(f, step, kMaxSkip3D);
@@ -3038,8 +3412,8 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                         th = nh;
                         tl = nl;
                         steps += (uint32_t)skip;
-                        c_steps += (uint32_t)skip;
-                        c_skipped += (uint32_t)skip;
+                        c_steps += one * (uint32_t)skip;
+                        c_skipped += one * (uint32_t)skip;
                         skip = 0;
                     }
                 }
@@ -3055,14 +3429,14 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                         status = GPIS_FLIGHT_STEP_LIMIT;
                         t_out = far_t;
                         t_end = {far_t, 0.0f};
-                        c_limit++;
+                        c_limit += one;
                         break;
                     }
                     if (skip == 0) break;
                     skip--;
                     steps++;
-                    c_steps++;
-                    c_skipped++;
+                    c_steps += one;
+                    c_skipped += one;
                     ff_add(th, tl, step);
                 }
             }
@@ -3078,13 +3452,13 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
             phase = PH_REFINE;
             if (CERT && !cert_fac(pf, fb, kPreciseBand, dfac)) {
                 steps--;
-                c_steps--;
+                c_steps -= one;
                 pf_precise = false;
                 phase = PH_MARCH_P;
                 pend = true;
             }
         } else if (phase == PH_REFINE) {
-            c_refine++;
+            c_refine += one;
             refine_iter++;
             bool hit = false;
             if (sg == sign0) {
@@ -3108,7 +3482,7 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
                 t_out = __fadd_rn(tprev.h, tprev.l);
                 v_out = 0.0f;
                 trans = 0.0f;
-                c_hits++;
+                c_hits += one;
             }
         } else {  // PH_FAR
             done = true;
@@ -3118,13 +3492,17 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
         }
         if (pend) {
             // (a value the certified pass took is never a precise one)
-            a.resume[fid] = pack_resume(th, tl, pf, steps, sign0, pf_precise && !CERT, phase, CERT);
-            if (queue_out) queue_push(queue_out, queue_len, fid);
+            if (lead) {
+                a.resume[fid] = pack_resume(th, tl, pf, steps, sign0, pf_precise && !CERT, phase, CERT);
+                if (queue_out) queue_push(queue_out, queue_len, fid);
+            }
             phase = PH_IDLE;
         } else if (done) {
-            write_status(a, fid, t_out, v_out, trans, steps, status | ((uint32_t)gpid << 8));
-            a.t_end[fid] = (double)t_end.h + (double)t_end.l;
-            if (!RESUME || CERT) a.resume[fid] = make_uint4(0u, 0u, 0u, 0u);
+            if (lead) {
+                write_status(a, fid, t_out, v_out, trans, steps, status | ((uint32_t)gpid << 8));
+                a.t_end[fid] = (double)t_end.h + (double)t_end.l;
+                if (!RESUME || CERT) a.resume[fid] = make_uint4(0u, 0u, 0u, 0u);
+            }
             phase = PH_IDLE;
         }
     }
@@ -3142,6 +3520,23 @@ __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
         atomicAdd(a.counters + 6, s6);
         atomicAdd(a.counters + 7, s7);
     }
+}
+
+template <class Eval, bool RESUME, bool CERT = false>
+__global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
+{
+    march_flights<Eval, RESUME, CERT>(a);
+}
+
+// The fast pass with two group sizes of one evaluator: batches of fewer than `few`
+// flights, which cannot fill the chip with small groups and wait for their longest
+// flight, take the larger.  The count is read on the device, so that rounds whose length
+// the host does not know choose too.
+template <class Wide, class Narrow>
+__global__ void __launch_bounds__(256, Narrow::kMinBlocks) k_march_sized(FlightArgs a, uint32_t few)
+{
+    if (live_n(a) < few) march_flights<Wide, false>(a);
+    else march_flights<Narrow, false>(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -3671,7 +4066,10 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
     // than one that scans every resume record in flight order (the uneven image batch
     // 512 against 496 ms)
     const bool certify = coop_plain && !a.precise_only;
-    if (!certify) b.queue = nullptr;
+    // stationary 3D media of up to 8 impulses per cell: lane groups, each of which loads
+    // its flight's record once for all its lanes, so the scattered order costs nothing
+    const bool group3 = a.three_d && a.max_oct == 1 && !a.any_ns && !a.any_gen3d && a.max_imp <= (uint32_t)kG3Imp;
+    if (!certify && !group3) b.queue = nullptr;
     if (b.any_cond || b.setup) {
         if (a.one_d) k_prepare<8><<<blocks, 128, 0, stream>>>(b);
         else k_prepare<4><<<blocks, 128, 0, stream>>>(b);
@@ -3681,9 +4079,8 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
     if (err != cudaSuccess) return err;
     // persistent grids: exactly the CTAs that are resident at once, never more
     // warps than flights
-    const uint32_t warps_needed = (a.n + 31) / 32;
-    const uint32_t ctas_needed = (warps_needed + 7) / 8;
-    auto grid = [&](const void *fn, size_t smem = 0, bool tuned = true) {
+    auto grid = [&](const void *fn, size_t smem = 0, bool tuned = true, uint32_t group = 1) {
+        const uint32_t ctas_needed = (uint32_t)(((uint64_t)a.n * group + 255) / 256);
         int per_sm = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, smem) != cudaSuccess || per_sm < 1)
             per_sm = 1;
@@ -3717,6 +4114,12 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
     } else if (coop) {
         const void *fn = (const void *)k_march<EvalCoop1D<8>, false>;
         k_march<EvalCoop1D<8>, false><<<grid(fn), 256, 0, stream>>>(b);
+    } else if (group3) {
+        const void *fn = (const void *)k_march_sized<EvalGroup3D<32>, EvalGroup3D<8>>;
+        cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemG3<8>);
+        if (e != cudaSuccess) return e;
+        k_march_sized<EvalGroup3D<32>, EvalGroup3D<8>>
+            <<<grid(fn, kSmemG3<8>, true, 32), 256, kSmemG3<8>, stream>>>(b, kG3Few);
     } else if (a.three_d && a.max_oct == 1 && !a.any_ns && !a.any_gen3d) {
         // 3D stationary single-octave media: the generic evaluator with step skipping
         const void *fn = (const void *)k_march<EvalSkip3D, false>;
@@ -3734,7 +4137,12 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
         k_march<EvalGeneric4, true, true><<<grid(fn, 0, false), 256, 0, stream>>>(b);
         b.queue_in = 2;
     }
-    if (a.one_d && !certify) {
+    if (group3) {
+        // few flights with long chains of precise evaluations: a warp each (40 009
+        // flights: 1.47 ms a batch against 1.54 with eight lanes each; 2 500: 0.42 / 0.54)
+        const void *fn = (const void *)k_march<EvalGroup3D<32>, true>;
+        k_march<EvalGroup3D<32>, true><<<grid(fn, kSmemG3<32>, false, 32), 256, kSmemG3<32>, stream>>>(b);
+    } else if (a.one_d && !certify) {
         const void *fn = (const void *)k_march<EvalGeneric4, true>;
         k_march<EvalGeneric4, true><<<grid(fn, 0, false), 256, 0, stream>>>(b);
     } else {
