@@ -66,6 +66,8 @@ struct FlightArgs {
     uint32_t prop_cap;          // most steps one evaluation skips before a proposed interval (0: 32)
     uint32_t fast_window;       // stationary 1D fast pass: 0 impulse window in shared memory, 1 in registers
     uint32_t precise_only;      // 1: no certified resume pass (every crossing on the precise evaluator)
+    uint32_t run_lo, run_hi;    // set by launch_flights: a march pass runs when its flight count, read on
+                                // the device, lies in [run_lo, run_hi)
     const uint32_t *n_dev;      // may be null: the live flight count in device memory (<= n,
                                 // which is then the capacity the grids are sized for)
     const float4 *proposal;     // may be null: per flight the proposed crossing interval
