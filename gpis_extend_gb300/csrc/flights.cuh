@@ -49,8 +49,9 @@ struct FlightArgs {
                                 // scan every flight): the flights the fast pass hands on, then
                                 // those the certified resume pass hands on
     int queue_in;               // set by launch_flights for each resume pass
-    float4 *setup;              // scratch, 4 per flight: the fast pass's per-flight set-up, written by
-                                // k_prepare when the stationary cooperative evaluator runs (else unused)
+    uint32_t setup_len;         // set by launch_flights: float4 per set-up record
+    float4 *setup;              // scratch, setup_len() per flight: the march passes' per-flight set-up,
+                                // written by k_prepare for batches of 1D media (else unused)
     unsigned long long *counters;  // gpis_counters block (8 x u64)
     int any_cond;               // some medium conditions (run the prepare kernel)
     int one_d;                  // all media use 1D noise
@@ -74,6 +75,15 @@ struct FlightArgs {
                                 // (t_a, t_b, miss probability, -); the fast pass may skip
                                 // further than its usual cap before t_a
 };
+
+// Batches of 1D media with up to 8 impulses per cell take the cooperative and lane-group
+// evaluators, whose flights start from the set-up record that k_prepare wrote: 4 float4
+// where every medium is stationary with one octave, 8 otherwise; 0: no record.
+inline uint32_t setup_len(bool one_d, uint32_t max_imp, uint32_t max_oct, bool any_ns, bool any_mr)
+{
+    if (!one_d || max_imp > 8u) return 0u;
+    return max_oct == 1u && !any_ns && !any_mr ? 4u : 8u;
+}
 
 // Per-flight features of the learned proposal (proposal.cu).
 cudaError_t launch_features(const DevMedium *media, int n_media, const gpis_flight_soa &in, uint32_t n, float *feat,

@@ -185,9 +185,9 @@ int derive_medium(const gpis_medium_desc &d, gpis::DevMedium &m)
         if (pow2) m.oct_pow2 |= 1u << k;
     }
     // The mean's slope bound for step skipping (SDFs are 1-Lipschitz; a linear mean
-    // has the slope of its scaled normal); not for multi-resolution media
+    // has the slope of its scaled normal)
     m.skip_mean_lip = -1.0f;
-    if (!multires) {
+    {
         switch (d.mean_kind) {
         case GPIS_MEAN_SPHERE: case GPIS_MEAN_TORUS: case GPIS_MEAN_TORUS_PLANE: m.skip_mean_lip = 1.0f; break;
         case GPIS_MEAN_HOMOGENEOUS: m.skip_mean_lip = 0.0f; break;
@@ -260,6 +260,7 @@ struct gpis_ctx {
     double *d_tend = nullptr;
     uint4 *d_resume = nullptr;
     float4 *d_setup = nullptr;
+    uint32_t setup_len = 0;                // float4 per flight of d_setup (gpis::setup_len)
     uint32_t *d_queue = nullptr;
     uint32_t *d_work = nullptr;
     unsigned long long *d_counters = nullptr;
@@ -337,7 +338,8 @@ int ensure_scratch(gpis_ctx *c, size_t n)
     CUDA_TRY(cudaMalloc(&c->d_cond, cap * sizeof(gpis::CondRec)), "allocate conditioning scratch");
     CUDA_TRY(cudaMalloc(&c->d_tend, cap * sizeof(double)), "allocate end-parameter scratch");
     CUDA_TRY(cudaMalloc(&c->d_resume, cap * sizeof(uint4)), "allocate resume scratch");
-    CUDA_TRY(cudaMalloc(&c->d_setup, cap * 4 * sizeof(float4)), "allocate set-up scratch");
+    if (c->setup_len)
+        CUDA_TRY(cudaMalloc(&c->d_setup, cap * c->setup_len * sizeof(float4)), "allocate set-up scratch");
     CUDA_TRY(cudaMalloc(&c->d_queue, cap * 2 * sizeof(uint32_t)), "allocate hand-off queues");
     c->cap = cap;
     return GPIS_OK;
@@ -457,6 +459,7 @@ int gpis_ctx_create(const gpis_medium_desc *media, int n_media, gpis_ctx **out)
             c->any_mr = c->any_mr || (m.flags & gpis::MF_MULTIRES) != 0u;
             c->any_gen3d = c->any_gen3d || gpis::general_3d(m);
         }
+        c->setup_len = gpis::setup_len(c->all_one_d, c->max_imp, c->max_oct, c->any_ns, c->any_mr);
         if (rc) break;
         if ((e = cudaMalloc(&c->d_media, host.size() * sizeof(gpis::DevMedium))) != cudaSuccess) { rc = cuda_fail(e, "allocate media"); break; }
         if ((e = cudaMemcpy(c->d_media, host.data(), host.size() * sizeof(gpis::DevMedium), cudaMemcpyHostToDevice)) != cudaSuccess) {
@@ -514,7 +517,7 @@ int submit_slice(gpis_ctx *ctx, const gpis_flight_soa *in, const gpis_result_soa
     a.t_end = ctx->d_tend + offset;
     a.work = work;
     a.resume = ctx->d_resume + offset;
-    a.setup = ctx->d_setup + 4 * offset;
+    a.setup = ctx->d_setup + (size_t)ctx->setup_len * offset;
     a.queue = ctx->d_queue + 2 * offset;
     a.counters = ctx->d_counters;
     a.any_cond = ctx->any_cond;
@@ -633,7 +636,7 @@ __attribute__((visibility("hidden"))) int gpis_internal_nee_live(gpis_ctx *ctx, 
 }
 
 // SM count, whether per-kernel profiling is on, and whether a flight batch runs the
-// prepare kernel (conditioning media, or the stationary cooperative fast pass's set-up)
+// prepare kernel (conditioning media, or the 1D passes' set-up records)
 int gpis_tune_set(gpis_ctx *ctx, uint32_t key, uint64_t value)
 {
     if (!ctx) return fail(GPIS_EINVAL, "null context");
@@ -672,11 +675,7 @@ __attribute__((visibility("hidden"))) int gpis_internal_ctx_info(gpis_ctx *ctx, 
     if (!ctx) return GPIS_EINVAL;
     if (num_sms) *num_sms = ctx->num_sms;
     if (profiling) *profiling = ctx->profiling ? 1 : 0;
-    if (prepare_runs) {
-        const bool coop_plain = ctx->all_one_d && ctx->max_imp <= 8 && ctx->max_oct == 1 && !ctx->any_ns &&
-                                !ctx->all_grid && !ctx->any_mr;
-        *prepare_runs = (ctx->any_cond || coop_plain) ? 1 : 0;
-    }
+    if (prepare_runs) *prepare_runs = (ctx->any_cond || ctx->setup_len) ? 1 : 0;
     return GPIS_OK;
 }
 

@@ -33,21 +33,14 @@ def test_gpu_3d_groups_match_oracle(n, impulses, kw):
 
 
 def test_gpu_3d_group_sizes_agree():
-    """Both group sizes on the same flights: decisions and hits are taken on the precise
-    values, so they agree bit for bit; a miss value is a sum in another order (24 terms of
-    magnitude below 1 within about 1e-6 of each other after the normalisation)."""
+    """Both group sizes on the same flights give the same records."""
     desc = medium_3d(8, context=abi.CTX_RENEWAL)
     prim = workloads.sphere_flights(10500, desc)
     idx = np.arange(0, prim.n, 3)
     with runtime.Context(desc) as ctx:
         many = ctx.trace_host(prim)[idx]
         few = ctx.trace_host(prim.subset(idx))
-    a, b = abi.unpack_results(many), abi.unpack_results(few)
-    for name in ("status", "steps", "hit", "t", "gp_id"):
-        assert np.array_equal(a[name], b[name]), name
-    hit = a["hit"]
-    assert np.array_equal(many[hit].view(np.uint32), few[hit].view(np.uint32))
-    assert np.abs(a["value"] - b["value"]).max() <= 2e-6
+    assert np.array_equal(many.view(np.uint32), few.view(np.uint32))
 
 
 MEDIA_1D = {
@@ -86,10 +79,84 @@ def test_gpu_1d_group_and_lane_passes_agree(precise):
         whole = ctx.trace_host(prim)
         parts = [ctx.trace_host(prim.subset(np.arange(k, k + 50_000))) for k in range(0, prim.n, 50_000)]
     part = np.concatenate(parts)
-    hit = abi.unpack_results(whole)["hit"]
-    assert hit.sum() > 200_000
-    assert np.array_equal(whole[hit].view(np.uint32), part[hit].view(np.uint32))
-    a, b = abi.unpack_results(whole), abi.unpack_results(part)
-    for name in ("status", "steps", "hit", "t", "gp_id"):
-        assert np.array_equal(a[name], b[name]), name
-    assert np.abs(a["value"] - b["value"]).max() <= 2e-6
+    assert abi.unpack_results(whole)["hit"].sum() > 200_000
+    assert np.array_equal(whole.view(np.uint32), part.view(np.uint32))
+
+
+@pytest.mark.parametrize("kind", ["sphere", "octaves", "multires", "nonstationary", "xy"])
+def test_gpu_1d_fast_passes_agree(kind):
+    """The fast passes on groups and on single lanes give the same records (misses too)."""
+    make, flights, half = MEDIA_1D[kind]
+    desc = make()
+    prim = flights(48_000, desc)
+    with runtime.Context(desc) as ctx:
+        whole = ctx.trace_host(prim)
+        parts = np.concatenate([ctx.trace_host(prim.subset(np.arange(k, k + 6000))) for k in range(0, prim.n, 6000)])
+        sec, _ = workloads.secondary_flights(prim, whole, desc, half=half)
+        two = abi.FlightBatch(2 * sec.n)
+        for name in ("origin_near", "dir_far", "seeds", "prev"):
+            getattr(two, name)[:] = np.concatenate([getattr(sec, name)] * 2)
+        whole2 = ctx.trace_host(two)
+        parts2 = np.concatenate([ctx.trace_host(sec.subset(np.arange(k, min(k + 6000, sec.n))))
+                                 for k in range(0, sec.n, 6000)])
+    assert np.array_equal(whole.view(np.uint32), parts.view(np.uint32))
+    assert two.n > 45_000 and np.array_equal(whole2[:sec.n].view(np.uint32), parts2.view(np.uint32))
+
+
+def torus_stationary(**kw):
+    return workloads.torus_plane_medium(nonstationary=False, octaves=1, **kw)
+
+
+@pytest.mark.parametrize("kind,n", [("octaves", 45001), ("multires", 45001), ("nonstationary", 46000), ("sphere", 40001),
+                                    ("torus", 40961), ("plane", 41003)])
+def test_gpu_1d_lane_passes_match_oracle(kind, n):
+    """Batches just above the limits of the group fast passes: the cooperative single-lane
+    passes, whose evaluations decide steps on both sides (the slope bound of several
+    octaves, of a nonstationary scale and of the multi-resolution grid; the second-order
+    reach of stationary media with a sphere, torus and linear mean)."""
+    if kind == "torus":
+        make, flights, half = torus_stationary, workloads.torus_flights, 2.0
+    elif kind == "plane":
+        make = lambda: workloads.sphere_medium(mean_kind=abi.MEAN_PLANE, mean_params=(0.0, 0.8, 0.6, 0.1))
+        flights, half = workloads.sphere_flights, 1.5
+    else:
+        make, flights, half = MEDIA_1D[kind]
+    desc = make()
+    prim = flights(n, desc)
+    with runtime.Context(desc) as ctx:
+        ctx.counters(reset=True)
+        rec = ctx.trace_host(prim)
+        cnt = ctx.counters(reset=True)
+        assert cnt["skipped_steps"] > 0.2 * cnt["steps"], cnt
+        rec_cpu, _ = flights_vs_oracle(desc, prim, rec, scene=half)
+        steps_gpu, steps_cpu = abi.unpack_results(rec)["steps"], abi.unpack_results(rec_cpu)["steps"]
+        assert np.mean(steps_gpu == steps_cpu) >= 0.9999
+        sec, _ = workloads.secondary_flights(prim, rec_cpu, desc, half=half)
+        if sec.n > 45000 or kind in ("sphere", "torus", "plane"):
+            flights_vs_oracle(desc, sec, ctx.trace_host(sec), scene=half)
+
+
+@pytest.mark.parametrize("far,step,max_steps", [(0.004, 0.01, 0), (3.0, 0.01, 37), (3.0, 0.75, 0), (3.0, 0.01, 300)])
+def test_gpu_reach_ends_with_the_march(far, step, max_steps):
+    """Reaches that pass farT or the step limit: the steps taken and the statuses are the
+    oracle's (flights shorter than a step, a limit inside the first reach, coarse steps)."""
+    desc = workloads.sphere_medium(step_size=step, min_step=1, max_steps=max_steps)
+    prim = workloads.sphere_flights(3000, desc)
+    prim.dir_far[:, 3] = np.minimum(prim.dir_far[:, 3], np.float32(far))
+    prim.dir_far[::7, 3] *= np.float32(0.37)
+    rec_cpu = oracle.trace_flights(desc, prim)
+    c = abi.unpack_results(rec_cpu)
+    with runtime.Context(desc) as ctx:
+        g = abi.unpack_results(ctx.trace_host(prim))
+    assert np.array_equal(g["status"], c["status"])
+    assert np.array_equal(g["steps"], c["steps"])
+    assert np.array_equal(g["hit"], c["hit"])
+    many = abi.FlightBatch(45_000)
+    idx = np.arange(45_000) % 3000
+    for name in ("origin_near", "dir_far", "seeds", "prev"):
+        getattr(many, name)[:] = getattr(prim, name)[idx]
+    with runtime.Context(desc) as ctx:
+        g = abi.unpack_results(ctx.trace_host(many))
+    assert np.array_equal(g["status"], c["status"][idx])
+    assert np.array_equal(g["steps"], c["steps"][idx])
+    assert np.array_equal(g["hit"], c["hit"][idx])
