@@ -146,24 +146,31 @@ __global__ void __launch_bounds__(128) k_gemm(Gemm g)
 }
 
 // ---- elementwise kernels ---------------------------------------------------------------
-// GRU inputs of every step, the globals part of the MLP input, h_0 = 0.
+// GRU inputs of every step, the globals part of the MLP input, h_0 = 0: one thread per
+// flight and part (a step's 16 inputs, the globals, h_0), 16-byte stores that run along
+// the flights.  (One thread per flight storing all 224 values by element took 42 us for
+// 8192 flights, 32 blocks of strided 2-byte stores.)
 __global__ void k_prep(const float *feat, uint32_t n, bf *xb, bf *ub, float *h0, bf *h0b)
 {
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
     if (m >= n) return;
     const float *f = feat + (size_t)m * NFEAT;
-    for (int j = 0; j < NHIST; ++j) {
-        bf *x = xb + ((size_t)j * n + m) * NIN;
-        x[0] = __float2bfloat16_rn(f[2 * j]);
-        x[1] = __float2bfloat16_rn(f[2 * j + 1]);
-        for (int c = 2; c < NIN; ++c) x[c] = __float2bfloat16_rn(0.0f);
-    }
-    bf *u = ub + (size_t)m * MLPIN;
-    for (int c = 0; c < 8; ++c) u[HID + c] = __float2bfloat16_rn(f[16 + c]);
-    for (int c = HID + 8; c < MLPIN; ++c) u[c] = __float2bfloat16_rn(0.0f);
-    for (int c = 0; c < HID; ++c) {
-        h0[(size_t)m * HID + c] = 0.0f;
-        h0b[(size_t)m * HID + c] = __float2bfloat16_rn(0.0f);
+    const int part = blockIdx.y;
+    const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
+    if (part < NHIST) {
+        uint4 *x = reinterpret_cast<uint4 *>(xb + ((size_t)part * n + m) * NIN);
+        x[0] = make_uint4(pack2f(f[2 * part], f[2 * part + 1]), 0u, 0u, 0u);
+        x[1] = zero;
+    } else if (part == NHIST) {
+        uint4 *u = reinterpret_cast<uint4 *>(ub + (size_t)m * MLPIN + HID);
+        u[0] = make_uint4(pack2f(f[16], f[17]), pack2f(f[18], f[19]), pack2f(f[20], f[21]), pack2f(f[22], f[23]));
+        u[1] = zero;
+    } else {
+        uint4 *a = reinterpret_cast<uint4 *>(h0 + (size_t)m * HID), *b = reinterpret_cast<uint4 *>(h0b + (size_t)m * HID);
+#pragma unroll
+        for (int c = 0; c < HID / 4; ++c) a[c] = zero;
+#pragma unroll
+        for (int c = 0; c < HID / 8; ++c) b[c] = zero;
     }
 }
 
@@ -197,18 +204,33 @@ __global__ void k_bias_gelu(float *a, const float *bias, uint32_t n, int width, 
     y[i] = __float2bfloat16_rn(gelu(v));
 }
 
-// the mixture's negative log-likelihood and its gradient w.r.t. the 32 outputs, / n
-__global__ void k_loss(float *o, const float *bias, const float2 *tgt, uint32_t n, float inv_n, float *dof, bf *dob,
-                       float *loss)
+// the mixture's negative log-likelihood, its gradient w.r.t. the 32 outputs, / n (BF16,
+// the GEMMs' operand), and that gradient's sum over the flights (the output bias's
+// gradient, from the unrounded values).  64 threads per block: one thread carries a
+// flight's whole mixture, and 256 left 8192 flights on 32 of the SMs.
+constexpr int kLossThreads = 64;
+__global__ void __launch_bounds__(kLossThreads) k_loss(float *o, const float *bias, const float2 *tgt, uint32_t n,
+                                                       float inv_n, bf *dob, float *loss, float *dbias)
 {
+    __shared__ float col[kLossThreads][NOUT + 1];
     const uint32_t m = blockIdx.x * blockDim.x + threadIdx.x;
     float nll = 0.0f;
+    for (int c = 0; c < NOUT; ++c) col[threadIdx.x][c] = 0.0f;
     if (m < n) {
-        float *x = o + (size_t)m * NOUT;
-        for (int c = 0; c < NOUT; ++c) x[c] += bias[c];
+        float x[NOUT];
+        const float4 *xr = reinterpret_cast<const float4 *>(o + (size_t)m * NOUT);
+#pragma unroll
+        for (int c = 0; c < NOUT / 4; ++c) {
+            const float4 v = xr[c];
+            x[4 * c] = v.x + bias[4 * c];
+            x[4 * c + 1] = v.y + bias[4 * c + 1];
+            x[4 * c + 2] = v.z + bias[4 * c + 2];
+            x[4 * c + 3] = v.w + bias[4 * c + 3];
+        }
         const float us = tgt[m].x;
         const bool hit = tgt[m].y != 0.0f;
         float g[NOUT];
+#pragma unroll
         for (int c = 0; c < NOUT; ++c) g[c] = 0.0f;
         const float ql = x[24];
         if (hit) {
@@ -246,59 +268,90 @@ __global__ void k_loss(float *o, const float *bias, const float2 *tgt, uint32_t 
             nll = softplus(-ql);
             g[24] = -sigm(-ql);
         }
+        uint4 *d = reinterpret_cast<uint4 *>(dob + (size_t)m * NOUT);
+#pragma unroll
         for (int c = 0; c < NOUT; ++c) {
-            const float v = g[c] * inv_n;
-            dof[(size_t)m * NOUT + c] = v;
-            dob[(size_t)m * NOUT + c] = __float2bfloat16_rn(v);
+            g[c] *= inv_n;
+            col[threadIdx.x][c] = g[c];
         }
+#pragma unroll
+        for (int c = 0; c < NOUT / 8; ++c)
+            d[c] = make_uint4(pack2f(g[8 * c], g[8 * c + 1]), pack2f(g[8 * c + 2], g[8 * c + 3]),
+                              pack2f(g[8 * c + 4], g[8 * c + 5]), pack2f(g[8 * c + 6], g[8 * c + 7]));
     }
-    // one atomic per warp
+    // one atomic per warp, and one per block and output
     for (int off = 16; off > 0; off >>= 1) nll += __shfl_xor_sync(0xffffffffu, nll, off);
     if ((threadIdx.x & 31) == 0) atomicAdd(loss, nll);
+    __syncthreads();
+    if (threadIdx.x < NOUT) {
+        float sum = 0.0f;
+#pragma unroll 8
+        for (int r = 0; r < kLossThreads; ++r) sum += col[r][threadIdx.x];
+        atomicAdd(dbias + threadIdx.x, sum);
+    }
 }
 
-// out[c] += sum over rows of x[m * ld + c], c < width
-__global__ void k_colsum(const float *x, uint32_t n, int width, long ld, float *out)
+// The backward elementwise kernels add up their layer's bias gradient on the way (the
+// sums over the flights of the unrounded FP32 gradients): 256 threads walk the rows, a
+// thread stays in its column, and a block adds its partial sums with one atomic per
+// column.  Separate column-sum kernels over FP32 copies of the gradients took 0.59 of the
+// 1.6 ms of a gradient over 8192 flights.
+constexpr unsigned kBackBlocks = 608;   // 4 blocks on each of the SMs
+
+// da = dy * gelu'(a) (BF16), dbias[c] += sum of da over the rows
+__global__ void __launch_bounds__(256) k_gelu_back(const float *dy, const float *a, uint32_t n, bf *dab, float *dbias)
 {
-    const int c = threadIdx.x % width;
-    const int rows_per = blockDim.x / width;
-    float s = 0.0f;
-    for (uint32_t m = blockIdx.x * rows_per + threadIdx.x / width; m < n; m += gridDim.x * rows_per)
-        s += x[(size_t)m * ld + c];
-    if ((int)threadIdx.x < rows_per * width) atomicAdd(out + c, s);
+    __shared__ float part[256];
+    const int c = threadIdx.x % WID;
+    float sum = 0.0f;
+    for (size_t m = (size_t)blockIdx.x * (256 / WID) + threadIdx.x / WID; m < n; m += (size_t)gridDim.x * (256 / WID)) {
+        const size_t i = m * WID + c;
+        const float v = dy[i] * gelu_grad(a[i]);
+        sum += v;
+        dab[i] = __float2bfloat16_rn(v);
+    }
+    part[threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.x < WID)
+        atomicAdd(dbias + c, (part[c] + part[WID + c]) + (part[2 * WID + c] + part[3 * WID + c]));
 }
 
-// da = dy * gelu'(a) (fp32 and bf16)
-__global__ void k_gelu_back(const float *dy, const float *a, uint32_t n, int width, float *daf, bf *dab)
+// one GRU step backward: gate gradients (BF16), dh * z, and the sums of the gate
+// gradients over the rows (b_ih: r, z, n; b_hh: r, z, n * r)
+__global__ void __launch_bounds__(256) k_gru_back(const float *dh, long ldh, const float *r_, const float *z_,
+                                                  const float *n_, const float *ghn_, const float *hprev, uint32_t n,
+                                                  bf *dgib, bf *dghb, float *dhpart, float *dbih, float *dbhh)
 {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n * (uint32_t)width) return;
-    const float v = dy[i] * gelu_grad(a[i]);
-    daf[i] = v;
-    dab[i] = __float2bfloat16_rn(v);
-}
-
-// one GRU step backward: gate gradients and dh * z
-__global__ void k_gru_back(const float *dh, long ldh, const float *r_, const float *z_, const float *n_,
-                           const float *ghn_, const float *hprev, uint32_t n, float *dgif, bf *dgib, float *dghf,
-                           bf *dghb, float *dhpart)
-{
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n * HID) return;
-    const uint32_t m = i / HID, c = i % HID;
-    const float d = dh[(size_t)m * ldh + c];
-    const float r = r_[i], z = z_[i], nn = n_[i], ghn = ghn_[i];
-    const float dz = d * (hprev[i] - nn) * z * (1.0f - z);
-    const float dn = d * (1.0f - z) * (1.0f - nn * nn);
-    const float dr = dn * ghn * r * (1.0f - r);
-    float *gi = dgif + (size_t)m * 3 * HID, *gh = dghf + (size_t)m * 3 * HID;
-    bf *gib = dgib + (size_t)m * 3 * HID, *ghb = dghb + (size_t)m * 3 * HID;
-    gi[c] = dr; gi[HID + c] = dz; gi[2 * HID + c] = dn;
-    gh[c] = dr; gh[HID + c] = dz; gh[2 * HID + c] = dn * r;
-    gib[c] = __float2bfloat16_rn(dr); gib[HID + c] = __float2bfloat16_rn(dz); gib[2 * HID + c] = __float2bfloat16_rn(dn);
-    ghb[c] = __float2bfloat16_rn(dr); ghb[HID + c] = __float2bfloat16_rn(dz);
-    ghb[2 * HID + c] = __float2bfloat16_rn(dn * r);
-    dhpart[i] = d * z;
+    __shared__ float4 part[256];
+    const int c = threadIdx.x % HID;
+    float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (size_t m = (size_t)blockIdx.x * (256 / HID) + threadIdx.x / HID; m < n; m += (size_t)gridDim.x * (256 / HID)) {
+        const size_t i = m * HID + c;
+        const float d = dh[m * ldh + c];
+        const float r = r_[i], z = z_[i], nn = n_[i], ghn = ghn_[i];
+        const float dz = d * (hprev[i] - nn) * z * (1.0f - z);
+        const float dn = d * (1.0f - z) * (1.0f - nn * nn);
+        const float dr = dn * ghn * r * (1.0f - r);
+        const float dnr = dn * r;
+        sum.x += dr; sum.y += dz; sum.z += dn; sum.w += dnr;
+        bf *gib = dgib + m * 3 * HID, *ghb = dghb + m * 3 * HID;
+        const bf br = __float2bfloat16_rn(dr), bz = __float2bfloat16_rn(dz);
+        gib[c] = br; gib[HID + c] = bz; gib[2 * HID + c] = __float2bfloat16_rn(dn);
+        ghb[c] = br; ghb[HID + c] = bz; ghb[2 * HID + c] = __float2bfloat16_rn(dnr);
+        dhpart[i] = d * z;
+    }
+    part[threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.x < 4 * HID) {
+        // thread q * 32 + c: sum q of column c over the block's eight rows
+        const int q = threadIdx.x / HID;
+        float v = 0.0f;
+#pragma unroll
+        for (int k = 0; k < 256 / HID; ++k) v += reinterpret_cast<const float *>(part + k * HID + c)[q];
+        if (q < 3) atomicAdd(dbih + q * HID + c, v);
+        if (q < 2) atomicAdd(dbhh + q * HID + c, v);
+        if (q == 3) atomicAdd(dbhh + 2 * HID + c, v);
+    }
 }
 
 // Adam on the FP32 master parameters, then their BF16 copies
@@ -927,7 +980,11 @@ __global__ void __launch_bounds__(128) k_tc_gemm_check(const bf *A, const bf *B,
 // columns) and commits them to an mbarrier, which every thread waits for (bounded) before
 // the next step overwrites the tiles.  The epilogue reads each thread's row (tcgen05.ld
 // 32x32b) and stores, adds or, with several K chunks, atomically adds it into C.
-// N % 16 == 0, N <= 128, K % 16 == 0.
+// N % 16 == 0, N <= 128, K % 16 == 0; the rows of C start on 16 bytes (ldc % 4 == 0).
+// What bounds it: latency (2 to 20 us a launch at 8192 flights for microseconds of work:
+// tensor-memory allocation, one or two staged chunks, the wait).  Staging the operands that
+// are contiguous along M or N by element in K order (2-byte loads 64 to 192 bytes apart)
+// made a weight gradient 28 to 32 us; by rows of eight K it reads along M and N.
 constexpr int TCG_KC = 64, TCG_NMAX = 128;
 constexpr uint32_t kTcgSmem = 128u * TCG_KC * 2u + 32u * TCG_KC * 2u;
 
@@ -956,7 +1013,6 @@ __global__ void __launch_bounds__(128) k_gemm_tc(Gemm g, uint32_t wait_limit, ui
     __syncthreads();
     umma::fence_after_sync();
     const uint32_t tmem = tslot;
-    const bf zero = __float2bfloat16_rn(0.0f);
     uint32_t phase = 0;
     bool fail = false, issued = false;
     for (int k16 = kt0; k16 < kt1; k16 += TCG_KC / 16) {
@@ -974,11 +1030,19 @@ __global__ void __launch_bounds__(128) k_gemm_tc(Gemm g, uint32_t wait_limit, ui
                 *reinterpret_cast<uint4 *>(sa + umma::tile_offset((uint32_t)r, (uint32_t)k, TCG_KC)) = v;
             }
         } else {
-            for (int i = (int)tid; i < 128 * kn; i += 128) {
-                const int r = i / kn, k = i - r * kn;
-                const long row = m0 + r;
-                const bf v = row < g.M ? g.A[row * g.lam + (kbase + k) * g.lak] : zero;
-                *reinterpret_cast<bf *>(sa + umma::tile_offset((uint32_t)r, (uint32_t)k, TCG_KC)) = v;
+            // (contiguous along M, the weight gradients' activations: a thread per row, so
+            // that the warp's loads run along M, eight K at a time for a 16-byte row)
+            const long row = m0 + (long)tid;
+            for (int k = 0; k < kn; k += 8) {
+                uint4 v = make_uint4(0u, 0u, 0u, 0u);
+                if (row < g.M) {
+                    const bf *a = g.A + row * g.lam + (kbase + k) * g.lak;
+                    bf e[8];
+#pragma unroll
+                    for (int q = 0; q < 8; ++q) e[q] = a[q * g.lak];
+                    v = make_uint4(pack2(e[0], e[1]), pack2(e[2], e[3]), pack2(e[4], e[5]), pack2(e[6], e[7]));
+                }
+                *reinterpret_cast<uint4 *>(sa + umma::tile_offset(tid, (uint32_t)k, TCG_KC)) = v;
             }
         }
         if (g.lbk == 1 && g.lbn % 8 == 0 && (reinterpret_cast<uintptr_t>(g.B) & 15u) == 0) {
@@ -989,10 +1053,14 @@ __global__ void __launch_bounds__(128) k_gemm_tc(Gemm g, uint32_t wait_limit, ui
                     *reinterpret_cast<const uint4 *>(g.B + (long)(n0 + c) * g.lbn + kbase + k);
             }
         } else {
-            for (int i = (int)tid; i < N * kn; i += 128) {
-                const int c = i / kn, k = i - c * kn;
-                *reinterpret_cast<bf *>(sb + umma::tile_offset((uint32_t)c, (uint32_t)k, TCG_KC)) =
-                    g.B[(kbase + k) * g.lbk + (long)(n0 + c) * g.lbn];
+            const int c = (int)tid % N;
+            for (int k = 8 * ((int)tid / N); k < kn; k += 8 * (128 / N)) {
+                const bf *b = g.B + (kbase + k) * g.lbk + (long)(n0 + c) * g.lbn;
+                bf e[8];
+#pragma unroll
+                for (int q = 0; q < 8; ++q) e[q] = b[q * g.lbk];
+                *reinterpret_cast<uint4 *>(sb + umma::tile_offset((uint32_t)c, (uint32_t)k, TCG_KC)) =
+                    make_uint4(pack2(e[0], e[1]), pack2(e[2], e[3]), pack2(e[4], e[5]), pack2(e[6], e[7]));
             }
         }
         umma::fence_async_smem();
@@ -1026,11 +1094,18 @@ __global__ void __launch_bounds__(128) k_gemm_tc(Gemm g, uint32_t wait_limit, ui
         umma::ld32(tmem + ((w * 32u) << 16), v);
         if (row < g.M) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) {
+            for (int j = 0; j < 32; j += 4) {
                 if (j < N) {
-                    if (g.ksplit > 1) atomicAdd(c + j, v[j]);
-                    else if (g.accumulate) c[j] += v[j];
-                    else c[j] = v[j];
+                    float4 *c4 = reinterpret_cast<float4 *>(c + j);
+                    const float4 w4 = make_float4(v[j], v[j + 1], v[j + 2], v[j + 3]);
+                    if (g.ksplit > 1) {
+                        atomicAdd(c4, w4);
+                    } else if (g.accumulate) {
+                        const float4 o4 = *c4;
+                        *c4 = make_float4(o4.x + w4.x, o4.y + w4.y, o4.z + w4.z, o4.w + w4.w);
+                    } else {
+                        *c4 = w4;
+                    }
                 }
             }
         }
@@ -1057,8 +1132,8 @@ struct gpis_proposal {
     bf *xb = nullptr, *ub = nullptr, *hb = nullptr, *y1 = nullptr, *y2 = nullptr, *y3 = nullptr, *dob = nullptr,
        *dab = nullptr, *dgib = nullptr, *dghb = nullptr;
     float *h = nullptr, *gi = nullptr, *gh = nullptr, *r = nullptr, *z = nullptr, *nn = nullptr, *ghn = nullptr,
-          *a1 = nullptr, *a2 = nullptr, *a3 = nullptr, *o = nullptr, *dof = nullptr, *dy = nullptr, *daf = nullptr,
-          *du = nullptr, *dgif = nullptr, *dghf = nullptr, *dh = nullptr, *loss = nullptr;
+          *a1 = nullptr, *a2 = nullptr, *a3 = nullptr, *o = nullptr, *dy = nullptr,
+          *du = nullptr, *dh = nullptr, *loss = nullptr;
     // fused inference: GPIS_PROPOSAL_KERNEL_*, resident blocks per SM of each form, and
     // the tensor-memory kernel's time-out flag (host-mapped, read by the next call)
     int kernel = GPIS_PROPOSAL_KERNEL_TC2;
@@ -1104,19 +1179,16 @@ int ensure_batch(gpis_proposal *p, uint32_t n)
     PTRY(palloc(p, p->ub, N * MLPIN), "allocate proposal activations");
     PTRY(palloc(p, p->hb, N * (NHIST + 1) * HID), "allocate proposal activations");
     PTRY(palloc(p, p->h, N * (NHIST + 1) * HID), "allocate proposal activations");
-    PTRY(palloc(p, p->gi, N * 3 * HID), "allocate proposal activations");
+    PTRY(palloc(p, p->gi, N * NHIST * 3 * HID), "allocate proposal activations");
     PTRY(palloc(p, p->gh, N * 3 * HID), "allocate proposal activations");
     for (float **q : {&p->r, &p->z, &p->nn, &p->ghn}) PTRY(palloc(p, *q, N * NHIST * HID), "allocate proposal activations");
-    for (float **q : {&p->a1, &p->a2, &p->a3, &p->dy, &p->daf}) PTRY(palloc(p, *q, N * WID), "allocate proposal activations");
+    for (float **q : {&p->a1, &p->a2, &p->a3, &p->dy}) PTRY(palloc(p, *q, N * WID), "allocate proposal activations");
     for (bf **q : {&p->y1, &p->y2, &p->y3, &p->dab}) PTRY(palloc(p, *q, N * WID), "allocate proposal activations");
     PTRY(palloc(p, p->o, N * NOUT), "allocate proposal activations");
-    PTRY(palloc(p, p->dof, N * NOUT), "allocate proposal activations");
     PTRY(palloc(p, p->dob, N * NOUT), "allocate proposal activations");
     PTRY(palloc(p, p->du, N * MLPIN), "allocate proposal activations");
-    PTRY(palloc(p, p->dgif, N * 3 * HID), "allocate proposal activations");
-    PTRY(palloc(p, p->dghf, N * 3 * HID), "allocate proposal activations");
-    PTRY(palloc(p, p->dgib, N * 3 * HID), "allocate proposal activations");
-    PTRY(palloc(p, p->dghb, N * 3 * HID), "allocate proposal activations");
+    PTRY(palloc(p, p->dgib, N * NHIST * 3 * HID), "allocate proposal activations");
+    PTRY(palloc(p, p->dghb, N * NHIST * 3 * HID), "allocate proposal activations");
     PTRY(palloc(p, p->dh, N * HID), "allocate proposal activations");
     PTRY(palloc(p, p->loss, 1), "allocate proposal activations");
     p->cap = n;
@@ -1145,14 +1217,14 @@ inline unsigned nb(size_t n, unsigned t = 256) { return (unsigned)((n + t - 1) /
 void forward(gpis_proposal *p, const float *feat, uint32_t n, cudaStream_t s)
 {
     const bf *wb = p->pb;
-    k_prep<<<nb(n), 256, 0, s>>>(feat, n, p->xb, p->ub, p->h, p->hb);
+    k_prep<<<dim3(nb(n, 128), NHIST + 2), 128, 0, s>>>(feat, n, p->xb, p->ub, p->h, p->hb);
+    // the input products of every step at once
+    gemm(p, s, p->xb, NIN, 1, wb + O_WIH, 1, NIN, p->gi, 3 * HID, NHIST * n, 3 * HID, NIN, 0);
     for (int j = 0; j < NHIST; ++j) {
-        const bf *x = p->xb + (size_t)j * n * NIN;
         const bf *hb = p->hb + (size_t)j * n * HID;
-        gemm(p, s, x, NIN, 1, wb + O_WIH, 1, NIN, p->gi, 3 * HID, n, 3 * HID, NIN, 0);
         gemm(p, s, hb, HID, 1, wb + O_WHH, 1, HID, p->gh, 3 * HID, n, 3 * HID, HID, 0);
         const size_t o = (size_t)j * n * HID;
-        k_gru_cell<<<nb((size_t)n * HID), 256, 0, s>>>(p->gi, p->gh, p->p, p->h + o, n, p->r + o, p->z + o, p->nn + o,
+        k_gru_cell<<<nb((size_t)n * HID), 256, 0, s>>>(p->gi + (size_t)j * n * 3 * HID, p->gh, p->p, p->h + o, n, p->r + o, p->z + o, p->nn + o,
                                                         p->ghn + o, p->h + o + (size_t)n * HID, p->hb + o + (size_t)n * HID,
                                                         j == NHIST - 1 ? p->ub : nullptr);
     }
@@ -1165,7 +1237,8 @@ void forward(gpis_proposal *p, const float *feat, uint32_t n, cudaStream_t s)
     gemm(p, s, p->y3, WID, 1, wb + O_W4, 1, WID, p->o, NOUT, n, NOUT, WID, 0);
 }
 
-int ksplit_for(uint32_t n) { return (int)std::max(1u, std::min(64u, n / 128)); }
+// K chunks of a weight gradient over k rows: 128 rows each, two staged steps
+int ksplit_for(size_t k) { return (int)std::max<size_t>(1, std::min<size_t>(512, k / 128)); }
 
 // loss and gradient of the mean loss into p->g (zeroed here)
 void backward(gpis_proposal *p, const float2 *tgt, uint32_t n, cudaStream_t s)
@@ -1175,39 +1248,37 @@ void backward(gpis_proposal *p, const float2 *tgt, uint32_t n, cudaStream_t s)
     const int ks = ksplit_for(n);
     cudaMemsetAsync(G, 0, N_PARAMS * sizeof(float), s);
     cudaMemsetAsync(p->loss, 0, sizeof(float), s);
-    k_loss<<<nb(n), 256, 0, s>>>(p->o, p->p + O_B4, tgt, n, 1.0f / (float)n, p->dof, p->dob, p->loss);
+    k_loss<<<nb(n, kLossThreads), kLossThreads, 0, s>>>(p->o, p->p + O_B4, tgt, n, 1.0f / (float)n, p->dob, p->loss,
+                                                        G + O_B4);
     // output layer
     gemm(p, s, p->dob, 1, NOUT, p->y3, WID, 1, G + O_W4, WID, NOUT, WID, n, 1, ks);
-    k_colsum<<<64, 256, 0, s>>>(p->dof, n, NOUT, NOUT, G + O_B4);
     gemm(p, s, p->dob, NOUT, 1, wb + O_W4, WID, 1, p->dy, WID, n, WID, NOUT, 0);
     // hidden layers 3, 2, 1
     const float *acts[3] = {p->a3, p->a2, p->a1};
     const bf *ins[3] = {p->y2, p->y1, p->ub};
     const int ow[3] = {O_W3, O_W2, O_W1}, ob[3] = {O_B3, O_B2, O_B1}, inw[3] = {WID, WID, MLPIN};
     for (int l = 0; l < 3; ++l) {
-        k_gelu_back<<<nb((size_t)n * WID), 256, 0, s>>>(p->dy, acts[l], n, WID, p->daf, p->dab);
+        k_gelu_back<<<std::min(nb((size_t)n * WID), kBackBlocks), 256, 0, s>>>(p->dy, acts[l], n, p->dab, G + ob[l]);
         gemm(p, s, p->dab, 1, WID, ins[l], inw[l], 1, G + ow[l], inw[l], WID, inw[l], n, 1, ks);
-        k_colsum<<<64, 256, 0, s>>>(p->daf, n, WID, WID, G + ob[l]);
         if (l < 2) gemm(p, s, p->dab, WID, 1, wb + ow[l], WID, 1, p->dy, WID, n, WID, WID, 0);
         else gemm(p, s, p->dab, WID, 1, wb + ow[l], MLPIN, 1, p->du, MLPIN, n, MLPIN, WID, 0);
     }
-    // GRU, through time
+    // GRU, through time; the steps' gate gradients stay, so that the weights' gradients
+    // are one product each over the rows of all steps
     const float *dh = p->du;
     long ldh = MLPIN;
     for (int j = NHIST - 1; j >= 0; --j) {
         const size_t o = (size_t)j * n * HID;
-        k_gru_back<<<nb((size_t)n * HID), 256, 0, s>>>(dh, ldh, p->r + o, p->z + o, p->nn + o, p->ghn + o, p->h + o,
-                                                        n, p->dgif, p->dgib, p->dghf, p->dghb, p->dh);
-        const bf *x = p->xb + (size_t)j * n * NIN;
-        const bf *hb = p->hb + o;
-        gemm(p, s, p->dgib, 1, 3 * HID, x, NIN, 1, G + O_WIH, NIN, 3 * HID, NIN, n, 1, ks);
-        gemm(p, s, p->dghb, 1, 3 * HID, hb, HID, 1, G + O_WHH, HID, 3 * HID, HID, n, 1, ks);
-        k_colsum<<<64, 192, 0, s>>>(p->dgif, n, 3 * HID, 3 * HID, G + O_BIH);
-        k_colsum<<<64, 192, 0, s>>>(p->dghf, n, 3 * HID, 3 * HID, G + O_BHH);
-        gemm(p, s, p->dghb, 3 * HID, 1, wb + O_WHH, HID, 1, p->dh, HID, n, HID, 3 * HID, 1);
+        bf *dgib = p->dgib + 3 * o, *dghb = p->dghb + 3 * o;
+        k_gru_back<<<std::min(nb((size_t)n * HID), kBackBlocks), 256, 0, s>>>(
+            dh, ldh, p->r + o, p->z + o, p->nn + o, p->ghn + o, p->h + o, n, dgib, dghb, p->dh, G + O_BIH, G + O_BHH);
+        if (j > 0) gemm(p, s, dghb, 3 * HID, 1, wb + O_WHH, HID, 1, p->dh, HID, n, HID, 3 * HID, 1);
         dh = p->dh;
         ldh = HID;
     }
+    const size_t rows = (size_t)NHIST * n;
+    gemm(p, s, p->dgib, 1, 3 * HID, p->xb, NIN, 1, G + O_WIH, NIN, 3 * HID, NIN, (int)rows, 1, ksplit_for(rows));
+    gemm(p, s, p->dghb, 1, 3 * HID, p->hb, HID, 1, G + O_WHH, HID, 3 * HID, HID, (int)rows, 1, ksplit_for(rows));
 }
 
 // Resident blocks per SM of a kernel with `dyn` bytes of dynamic shared memory (opted in
