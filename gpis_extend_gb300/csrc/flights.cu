@@ -991,7 +991,8 @@ __device__ __forceinline__ CondRec make_condition(const DevMedium &m, const Flig
 // eight: {frame normal, scale at the origin}, {step, t0, seed, flags}, two of skip
 // constants (skip_consts), then value scales, gradient scales along the ray and origin
 // coordinates of up to four octaves, {the origin's level weights, -, -}.
-enum : uint32_t { SF_VALID = 1u, SF_COND = 2u, SF_FIRST = 4u };
+enum : uint32_t { SF_VALID = 1u, SF_COND = 2u, SF_FIRST = 4u, SF_DIRECT = 8u };
+__device__ __forceinline__ bool t_direct_ok(float t0, float step, float far_t);
 
 __device__ __forceinline__ void skip_params(const DevMedium &m, const float d[3], float sigma, bool cond, float vs,
                                             float gsz, float step, float &lip, float &j0, float &j1)
@@ -1117,7 +1118,8 @@ __device__ __forceinline__ void prepare_one(const FlightArgs &a, uint32_t i)
     float step = __fdiv_rn(__fsub_rn(fl.far_t, fl.near_t), (float)m.min_step);
     if (m.step_size < step) step = m.step_size;
     const float t0 = __fadd_rn(fl.near_t, __fmul_rn(step, fl.jitter));
-    const uint32_t flags = SF_VALID | (cond ? SF_COND : 0u) | ((fl.flags & GPIS_FLAG_FIRST_SCATTER) ? SF_FIRST : 0u);
+    const uint32_t flags = SF_VALID | (cond ? SF_COND : 0u) | ((fl.flags & GPIS_FLAG_FIRST_SCATTER) ? SF_FIRST : 0u) |
+                           (t_direct_ok(t0, step, fl.far_t) ? SF_DIRECT : 0u);
     if (general) {
         float vs[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gz[4] = {0.0f, 0.0f, 0.0f, 0.0f}, oz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         float ls_o = 1.0f;
@@ -1153,12 +1155,45 @@ __device__ __forceinline__ void prepare_one(const FlightArgs &a, uint32_t i)
 // MINB blocks of 128 per SM: 8 (at most 64 registers) for batches of 1D media, 1.14
 // against 1.38 ms per bench step at 4 blocks and 128 registers (the precise
 // conditioning's FP64 work needs the warps); 4 when 3D media are present, whose 27-cell
-// evaluations spill heavily at 64 registers
+// evaluations spill heavily at 64 registers.
+//
+// A block takes its 128 flights conditioned ones first: the conditioning is nearly all of
+// a thread's work, and in a wavefront's queue, where conditioned and first flights come in
+// no order, half of the lanes waited for the others (half of the flights
+// conditioned: 0.20 -> 0.16 ms per million).
 template <int MINB>
 __global__ void __launch_bounds__(128, MINB) k_prepare(FlightArgs a)
 {
+    __shared__ uint32_t conds[4];
+    __shared__ uint8_t order[128];
     const uint32_t n = live_n(a);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) prepare_one(a, i);
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    for (uint32_t base = blockIdx.x * 128u; base < n; base += gridDim.x * 128u) {
+        const uint32_t i = base + tid;
+        bool cond = false;
+        if (i < n) {
+            bool mok;
+            const DevMedium &m = *medium_of(a, i, mok);
+            cond = (m.flags & MF_COND) && !(a.seeds[i].z & GPIS_FLAG_FIRST_SCATTER);
+        }
+        const unsigned mask = __ballot_sync(FULL, cond);
+        if (lane == 0) conds[warp] = mask;
+        __syncthreads();
+        uint32_t before = 0, total = 0;
+#pragma unroll
+        for (uint32_t w = 0; w < 4; ++w) {
+            const uint32_t c = (uint32_t)__popc(conds[w]);
+            before += w < warp ? c : 0u;
+            total += c;
+        }
+        before += (uint32_t)__popc(mask & ((1u << lane) - 1u));     // conditioned flights before this one
+        order[cond ? before : total + tid - before] = (uint8_t)tid;
+        __syncthreads();
+        const uint32_t mine = base + order[tid];
+        if (mine < n) prepare_one(a, mine);
+        // (warps that are done leave the block unless it goes on)
+        if (n - base > gridDim.x * 128u) __syncthreads();
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -1272,7 +1307,7 @@ __device__ __forceinline__ void lane_field_setup(LaneField &L, const DevMedium &
 // direction streams; false where the record says that the flight is not valid.
 struct LaneStart {
     float step, t0, curv, j0, j1, dn;
-    bool first;
+    bool first, direct;
 };
 template <int LEN>
 __device__ __forceinline__ bool lane_field_load(LaneField &L, const DevMedium &m, const float4 *s, const float4 &on,
@@ -1282,6 +1317,7 @@ __device__ __forceinline__ bool lane_field_load(LaneField &L, const DevMedium &m
     const uint32_t flags = __float_as_uint(LEN == 8 ? b.w : e.y);
     if (!(flags & SF_VALID)) return false;
     st.first = (flags & SF_FIRST) != 0;
+    st.direct = (flags & SF_DIRECT) != 0;
 #pragma unroll
     for (int k = 0; k < 3; ++k) L.li[k] = m.l_inv[k];
     L.o[0] = on.x; L.o[1] = on.y; L.o[2] = on.z;
@@ -2753,7 +2789,9 @@ __device__ __forceinline__ float fast_share(const LaneField &L, const FastPoint 
 // machine and the coordinates in eight lanes, so long queues, which fill the chip with
 // single lanes, take those: about 0.55 of the flights cross, a fifth of these stay
 // uncertified, and the lines lie between the measured sizes where the two cross.
-constexpr uint32_t kFewCertified = 100000, kFewPrecise = 200000;
+// (Several octaves since the set-up records: 300 007 flights 9 503 / 10 935, 60 013 on the
+// multi-resolution grid 4 392 / 5 818.)
+constexpr uint32_t kFewCertified = 100000, kFewPrecise = 200000, kFewPreciseGeneral = 1000000;
 // Fast passes the same way: plain media, 509 flights 159 / 253, 20 000 273 / 364, 65 537
 // 484 / 444, 262 144 1 423 / 867; three octaves, 10 000 2 988 / 4 308, 30 000 4 742 / 5 084,
 // 100 000 8 906 / 6 054; multi-resolution, 20 000 2 606 / 3 419, 60 013 5 296 / 4 818.
@@ -2950,7 +2988,8 @@ struct EvalGroup1D {
         return pair_sum();
     }
 
-    __device__ __forceinline__ float certified(const LaneField &L, float px, float py, float pz, int &id, float &margin)
+    __device__ __forceinline__ float certified(const LaneField &L, float px, float py, float pz, int &id, float &margin,
+                                               bool = true)
     {
         return value_1d_cert(L, px, py, pz, id, [&](float z, uint32_t seed, float ls) {
             return raw_sum<true>(*L.m, 0, z, seed, ls, &margin);
@@ -3001,88 +3040,183 @@ struct EvalGroup1D {
     }
 };
 
-// 1D evaluator with the three-cell impulse window in registers and a
-// warp-cooperative refill: the lanes whose query entered a new cell are
-// gathered by a ballot and the whole warp generates their cells, one impulse per
-// lane (the jump-ahead PCG draws any impulse of a cell independently), 32/NMAX
-// cells per pass; shuffles deliver each cell into its owner's registers.  Every
-// lane of the warp must call value() (idle lanes pass live = false).
-// SM: the three-cell window lives in dynamic shared memory as a ring of slots
-// (kSmem1D bytes per 256-thread block, float4 rows per lane as EvalCoopOct lays
-// them out) instead of 24 registers per lane; a one-cell move then refills one
-// slot without shifting the others.
-constexpr int kC1Threads = 256;
-constexpr size_t kSmem1D = (size_t)3 * 8 * sizeof(float) * kC1Threads;
+// Windows in shared memory: the impulses of the three cells around the query, per octave
+// a ring of three slots of 8 floats (position with the weight's sign in the sign bit) for
+// each lane, laid out [octave][cell slot][k / 4][lane] in float4 so that a warp's loads are
+// contiguous.  A ring index turns a one-cell move into one refill.
+constexpr int kWinThreads = 256;
+constexpr int kWinList = 64;        // listed cells per warp and round
+constexpr size_t kSmemList = (size_t)kWinList * (kWinThreads / 32) * sizeof(uint4);
+constexpr size_t smem_window(uint32_t octaves)
+{
+    return kSmemList + (size_t)octaves * 3 * 8 * sizeof(float) * kWinThreads;
+}
 
+__device__ __forceinline__ int window_place(int tid, int o, int slot) { return ((o * 3 + slot) * 2 * kWinThreads + tid) << 2; }
+
+// Logical cell j (0: ci - 1, 1: ci, 2: ci + 1) of octave o sits in slot (rot + j) mod 3,
+// rot two bits per octave.  A query that entered cell ci: the ring turned (up: the old
+// middle becomes the low cell), and which cells it needs as two bits: 1 the one above, 2 the
+// one below, 3 all three.
+__device__ __forceinline__ uint32_t window_turn(int o, int ci, bool ok, int &base, uint32_t &rot, int &count)
+{
+    const bool up = ok && ci == base + 1, down = ok && ci == base - 1;
+    int r = (rot >> (2 * o)) & 3u;
+    r = up ? (r == 2 ? 0 : r + 1) : (down ? (r == 0 ? 2 : r - 1) : 0);
+    rot = (rot & ~(3u << (2 * o))) | ((uint32_t)r << (2 * o));
+    base = ci;
+    count += up || down ? 1 : 3;
+    return (up ? 1u : (down ? 2u : 3u)) << (2 * o);
+}
+
+// The cells that a warp's lanes need, of every octave, are listed in shared memory and
+// drawn four at a time, eight lanes each, straight into their owners' slots.  kinds: two
+// bits per octave (window_turn), count: how many cells they are.  Every lane calls.
+template <int NOCT>
+__device__ __forceinline__ void window_fill(uint4 *list, float *cbase, const PcgJump *sj, uint32_t kinds, int count,
+                                            const int (&base)[NOCT], uint32_t rot, const uint32_t (&seeds)[NOCT],
+                                            uint32_t n_imp)
+{
+    const int lane = threadIdx.x & 31;
+    unsigned pend = __ballot_sync(FULL, count > 0);
+    while (pend) {
+        const bool mine = (pend >> lane) & 1u;
+        int incl = mine ? count : 0;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(FULL, incl, o);
+            if (lane >= o) incl += v;
+        }
+        // (a lane lists at most 12 cells, so the first that waits always fits)
+        const bool go = mine && incl <= kWinList;
+        const unsigned gm = __ballot_sync(FULL, go);
+        const int total = __shfl_sync(FULL, incl, 31 - __clz(gm));
+        if (go) {
+            uint4 *to = list + (incl - count);
+#pragma unroll
+            for (int o = 0; o < NOCT; ++o) {
+                const uint32_t kind = (kinds >> (2 * o)) & 3u;
+                if (!kind) continue;
+                const int r = (rot >> (2 * o)) & 3u;
+                const int s1 = r == 2 ? 0 : r + 1, s2 = r == 0 ? 2 : r - 1;
+                if (kind & 1u) *to++ = make_uint4((uint32_t)base[o] + 1u, seeds[o], window_place(threadIdx.x, o, s2), n_imp);
+                if (kind & 2u) *to++ = make_uint4((uint32_t)base[o] - 1u, seeds[o], window_place(threadIdx.x, o, r), n_imp);
+                if (kind == 3u) *to++ = make_uint4((uint32_t)base[o], seeds[o], window_place(threadIdx.x, o, s1), n_imp);
+            }
+        }
+        __syncwarp();
+        const int k = lane & 7;
+        for (int e = lane >> 3; e < total; e += 4) {
+            const uint4 q = list[e];
+            float v = kNoImpulse;
+            if ((uint32_t)k < q.w) {
+                const uint32_t s = xxhash2(q.x, q.y) + 1u;
+                const uint32_t r1 = pcg_draw(sj[2 + 2 * k], s);
+                const uint32_t r2 = pcg_draw(sj[3 + 2 * k], s);
+                v = __uint_as_float(__float_as_uint(unit_float(r1)) | (~r2 & 0x80000000u));
+            }
+            cbase[q.z + (k >> 2) * (4 * kWinThreads) + (k & 3)] = v;
+        }
+        __syncwarp();
+        pend &= ~gm;
+    }
+}
+
+// 1D evaluator of stationary single-octave media.  SM: the window in shared memory; else in
+// registers with a warp-cooperative refill: the lanes whose query entered a new cell are
+// gathered by a ballot and the whole warp generates their cells, one impulse per lane (the
+// jump-ahead PCG draws any impulse of a cell independently), 32/NMAX cells per pass;
+// shuffles deliver each cell into its owner's registers.  Every lane of the warp must call
+// value() (idle lanes pass live = false).
 template <int NMAX, bool GRID = false, bool SM = false>
 struct EvalCoop1D {
     static constexpr bool kCollective = true;
     static constexpr int kGroup = 1;
-    // CTAs per SM for the stationary analytic-mean kernel: with the window in shared
-    // memory 3 (80 registers; 14.34 ms per bench step against 14.72 for 4 CTAs at 64
-    // registers, whose spills feed long-scoreboard stalls, and 15.44 for 2 at 128),
-    // with the window in registers 4 (64 registers, 2 % faster than 2 CTAs at 128
-    // despite spills); the grid variant keeps 2
+    // CTAs per SM: with the window in shared memory 3 (80 registers), in registers 4 (64); a
+    // grid mean's eight voxels want 2 (128; 500 009 flights 1.40 ms a batch, 1.75 with 3)
     static constexpr int kMinBlocks = GRID ? 2 : (SM ? 3 : 4);
     static constexpr int kSetup = 4;
     static constexpr bool kSkip = true;
     float cache[SM ? 1 : 3][SM ? 1 : NMAX];
-    int base;
+    int base[1];
     bool valid;
     const PcgJump *sj;      // the jump table in shared memory
     float *cbase;           // SM: the window's shared memory
+    uint4 *list;            // SM: the warp's listed cells
     float slope;            // the derivative of the normalized noise in the iso coordinate
-    int rot;                // SM: logical cell j (0: ci - 1, 1: ci, 2: ci + 1) sits in slot (rot + j) mod 3
+    uint32_t rot;           // SM: the ring's turn
 
-    __device__ __forceinline__ void reset() { valid = false; base = 0; rot = 0; }
+    __device__ __forceinline__ void reset() { valid = false; base[0] = 0; rot = 0u; }
     __device__ __forceinline__ void bind(const PcgJump *t)
     {
         sj = t;
         if (SM) {
             extern __shared__ float4 dsm_c1[];
-            cbase = reinterpret_cast<float *>(dsm_c1);
+            list = reinterpret_cast<uint4 *>(dsm_c1) + (threadIdx.x >> 5) * kWinList;
+            cbase = reinterpret_cast<float *>(dsm_c1) + kSmemList / sizeof(float);
         }
-    }
-    __device__ __forceinline__ float *slot_ptr(int tid, int slot, int k) const
-    {
-        return cbase + (((slot * 2 + (k >> 2)) * kC1Threads + tid) << 2) + (k & 3);
     }
 
-    // SM: cooperative generation of one cell per requesting lane, each impulse written
-    // by the lane that draws it straight into the owner's ring slot
-    __device__ __forceinline__ void fill_sm(bool need, int cell, int slot, const LaneField &L, int lane)
+    // SM: the window around the coordinate z; its fraction in the cell
+    __device__ __forceinline__ float locate(const LaneField &L, float z, uint32_t &refills, bool live)
     {
-        unsigned mask = __ballot_sync(FULL, need);
-        const int rq = lane >> 3;
-        const int k = lane & 7;
-        const int warp0 = threadIdx.x & ~31;
-        while (mask) {
-            unsigned pass = 0u, mm = mask;
+        const float tg = __fdiv_rn(z, L.kr);
+        const float fl = floorf(tg);
+        const int ci = (int)fl;
+        uint32_t kinds = 0u;
+        int count = 0;
+        if (live && (!valid || ci != base[0])) {
+            kinds = window_turn(0, ci, valid, base[0], rot, count);
+            valid = true;
+        }
+        refills += (uint32_t)count;
+        const uint32_t seeds[1] = {L.seed};
+        window_fill<1>(list, cbase, sj, kinds, count, base, rot, seeds, L.n_imp);
+        return __fsub_rn(tg, fl);
+    }
+
+    // SM: f(term) of the 24 terms in the order of cells and impulses: distance in cells and
+    // signed value (0 out of reach)
+    template <class F>
+    __device__ __forceinline__ void each_term(float frac, float kexp, F f) const
+    {
+        const int s0 = (int)rot, s1 = s0 == 2 ? 0 : s0 + 1, s2 = s0 == 0 ? 2 : s0 - 1;
 #pragma unroll
-            for (int r = 0; r < 4; ++r) {
-                pass |= mm & (0u - mm);
-                mm &= mm - 1u;
-            }
-            mask = mm;
-            unsigned pm = pass;
-            for (int r = 0; r < rq; ++r) pm &= pm - 1u;
-            const int owner = pm ? __ffs(pm) - 1 : 0;
-            const int ocell = __shfl_sync(FULL, cell, owner);
-            const uint32_t oseed = __shfl_sync(FULL, L.seed, owner);
-            const int oslot = __shfl_sync(FULL, slot, owner);
-            const uint32_t onimp = __shfl_sync(FULL, L.n_imp, owner);
-            if (pm != 0u) {
-                float v = kNoImpulse;
-                if ((uint32_t)k < onimp) {
-                    const uint32_t s = xxhash2((uint32_t)ocell, oseed) + 1u;
-                    const uint32_t r1 = pcg_draw(sj[2 + 2 * k], s);
-                    const uint32_t r2 = pcg_draw(sj[3 + 2 * k], s);
-                    v = __uint_as_float(__float_as_uint(unit_float(r1)) | (~r2 & 0x80000000u));
+        for (int c = 0; c < 3; ++c) {
+            const float tl = __fsub_rn(frac, (float)(c - 1));
+            const float4 *row = reinterpret_cast<const float4 *>(cbase + window_place(threadIdx.x, 0, c == 0 ? s0 : (c == 1 ? s1 : s2)));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                const float4 q4 = row[h * kWinThreads];
+                const float qs[4] = {q4.x, q4.y, q4.z, q4.w};
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float tp = __fsub_rn(tl, fabsf(qs[j]));
+                    const float e = ex2_approx(kexp * (tp * tp));
+                    const float w = __uint_as_float(__float_as_uint(e) | (__float_as_uint(qs[j]) & 0x80000000u));
+                    f(j, tp, fabsf(tp) < 1.0f ? w : 0.0f);
                 }
-                *slot_ptr(warp0 + owner, oslot, k) = v;
             }
         }
-        __syncwarp();
+    }
+
+    // the certified pass's value (value_1d_cert): noise1d_generic's order of the sum, and the
+    // margin to the nearest support edge or cell face
+    __device__ __forceinline__ float certified(const LaneField &L, float px, float py, float pz, int &id, float &margin,
+                                               bool live)
+    {
+        static_assert(SM, "the certified pass keeps its windows in shared memory");
+        return value_1d_cert(L, px, py, pz, id, [&](float z, uint32_t, float) {
+            uint32_t refills = 0u;
+            const float frac = locate(L, z, refills, live);
+            float mg = fminf(frac, 1.0f - frac), sv = 0.0f;
+            each_term(frac, L.kexp, [&](int, float tp, float w) {
+                mg = fminf(mg, fabsf(fabsf(tp) - 1.0f));
+                sv = __fadd_rn(sv, w);
+            });
+            margin = mg - 0x1p-19f * (fabsf(__fdiv_rn(z, L.kr)) + 1.0f);
+            return sv;
+        });
     }
 
     template <int S>
@@ -3133,51 +3267,22 @@ struct EvalCoop1D {
         if (on_grid) grid_fetch(*L.m, px, py, pz, tap);
         const float z = ray_coord(L.li, L.n, px, py, pz);
         const float kexp = L.kexp, inv_norm = L.inv_norm;
-        const float tg = __fdiv_rn(z, L.kr);
-        const float fl = floorf(tg);
-        const float frac = __fsub_rn(tg, fl);
-        const int ci = (int)fl;
-        const bool changed = live && (!valid || ci != base);
-        const bool up = changed && valid && ci == base + 1;
-        const bool down = changed && valid && ci == base - 1;
-        const bool full = changed && !up && !down;
         float acc0 = 0.0f, acc1 = 0.0f, der0 = 0.0f, der1 = 0.0f;   // (der: sum of w e tp)
         if constexpr (SM) {
-            int r = rot;
-            if (up) r = r == 2 ? 0 : r + 1;          // the old middle becomes the low cell
-            if (down) r = r == 0 ? 2 : r - 1;
-            if (full) r = 0;
-            const int s0 = r, s1 = r == 2 ? 0 : r + 1, s2 = r == 0 ? 2 : r - 1;
-            fill_sm(full || down, ci - 1, s0, L, lane);
-            fill_sm(full, ci, s1, L, lane);
-            fill_sm(full || up, ci + 1, s2, L, lane);
-            if (changed) {
-                base = ci;
-                rot = r;
-                valid = true;
-                refills += full ? 3u : 1u;
-            }
-#pragma unroll
-            for (int c = 0; c < 3; ++c) {
-                const float tl = __fsub_rn(frac, (float)(c - 1));
-                const int slot = c == 0 ? s0 : (c == 1 ? s1 : s2);
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    const float4 q4 = *reinterpret_cast<const float4 *>(slot_ptr(threadIdx.x, slot, 4 * h));
-                    const float qs[4] = {q4.x, q4.y, q4.z, q4.w};
-#pragma unroll
-                    for (int j = 0; j < 4; ++j) {
-                        const float sv = qs[j];
-                        const float tp = __fsub_rn(tl, fabsf(sv));
-                        const float e = ex2_approx(kexp * (tp * tp));
-                        float w = __uint_as_float(__float_as_uint(e) | (__float_as_uint(sv) & 0x80000000u));
-                        w = fabsf(tp) < 1.0f ? w : 0.0f;
-                        if (j & 1) { acc1 += w; der1 += w * tp; }
-                        else { acc0 += w; der0 += w * tp; }
-                    }
-                }
-            }
+            const float frac = locate(L, z, refills, live);
+            each_term(frac, kexp, [&](int j, float tp, float w) {
+                if (j & 1) { acc1 += w; der1 += w * tp; }
+                else { acc0 += w; der0 += w * tp; }
+            });
         } else {
+            const float tg = __fdiv_rn(z, L.kr);
+            const float fl = floorf(tg);
+            const float frac = __fsub_rn(tg, fl);
+            const int ci = (int)fl;
+            const bool changed = live && (!valid || ci != base[0]);
+            const bool up = changed && valid && ci == base[0] + 1;
+            const bool down = changed && valid && ci == base[0] - 1;
+            const bool full = changed && !up && !down;
             if (up) {
 #pragma unroll
                 for (int k = 0; k < NMAX; ++k) { cache[0][k] = cache[1][k]; cache[1][k] = cache[2][k]; }
@@ -3190,7 +3295,7 @@ struct EvalCoop1D {
             fill_slot<1>(full, ci, L, lane);
             fill_slot<2>(full || up, ci + 1, L, lane);
             if (changed) {
-                base = ci;
+                base[0] = ci;
                 valid = true;
                 refills += full ? 3u : 1u;
             }
@@ -3226,24 +3331,14 @@ struct EvalCoop1D {
 
 // 1D evaluator for media with several octaves, a nonstationary length scale or the
 // multi-resolution grid (whose two levels count as octaves here): each octave's
-// three-cell impulse window (8 impulses per cell) lives in shared memory, 24 floats per
-// lane and octave, laid out [octave][cell slot][k / 4][lane] in float4 so that a warp's
-// loads are contiguous.  A ring index per octave turns a one-cell move into one refill.
-// The cells that the warp's lanes need, of every octave, are listed in shared memory and
-// drawn four at a time, eight lanes each.  Every lane of the warp must call value().
+// three-cell impulse window lives in shared memory, and the cells of all octaves are drawn
+// together (window_fill).  Every lane of the warp must call value().
 //
 // What bounds it: issue slots and the instruction cache.  Drawing per octave and slot
 // (nine ballots and loops per evaluation), taking the skip bound's per-flight terms and
 // the origin's coordinates again at every evaluation (about 70 IEEE divisions) and the
 // flight's set-up inside the march cost 2 540 instructions per lane and evaluation.
 constexpr int kOctMax = 4;
-constexpr int kOctThreads = 256;
-constexpr int kOctList = 64;        // listed cells per warp and round
-constexpr size_t kSmemOctList = (size_t)kOctList * (kOctThreads / 32) * sizeof(uint4);
-constexpr size_t smem_oct(uint32_t octaves)
-{
-    return kSmemOctList + (size_t)octaves * 3 * 8 * sizeof(float) * kOctThreads;
-}
 
 struct EvalCoopOct {
     static constexpr bool kCollective = true;
@@ -3251,10 +3346,10 @@ struct EvalCoopOct {
     static constexpr int kMinBlocks = 2;
     static constexpr int kSetup = 8;
     static constexpr bool kSkip = false;
-    float *cbase;           // float index ((o * 3 + slot) * 8 + k) maps to cbase[(((o*3+slot)*2 + k/4)*256 + tid)*4 + k%4]
-    uint4 *list;            // the warp's listed cells: cell, seed, place of impulse 0, impulses
+    float *cbase;
+    uint4 *list;
     int base[kOctMax];
-    uint32_t rot;           // two bits per octave: logical cell j (0: ci - 1, 1: ci, 2: ci + 1) sits in slot (rot + j) mod 3
+    uint32_t rot;
     uint32_t valid;         // bit o: octave o's window is filled
     uint32_t level;         // multi-resolution: the lower level's seed offset of the windows
     const PcgJump *sj;
@@ -3264,59 +3359,9 @@ struct EvalCoopOct {
     __device__ __forceinline__ void bind(const PcgJump *t)
     {
         extern __shared__ float4 dsm_oct[];
-        list = reinterpret_cast<uint4 *>(dsm_oct) + (threadIdx.x >> 5) * kOctList;
-        cbase = reinterpret_cast<float *>(dsm_oct) + kSmemOctList / sizeof(float);
+        list = reinterpret_cast<uint4 *>(dsm_oct) + (threadIdx.x >> 5) * kWinList;
+        cbase = reinterpret_cast<float *>(dsm_oct) + kSmemList / sizeof(float);
         sj = t;
-    }
-    static __device__ __forceinline__ int place(int tid, int o, int slot) { return ((o * 3 + slot) * 2 * kOctThreads + tid) << 2; }
-
-    // draws the cells that the lanes ask for: kind (two bits per octave) 1 the cell above
-    // the new centre, 2 the one below, 3 all three; count their number
-    __device__ __forceinline__ void fill(uint32_t kinds, int count, const LaneField &L, const uint32_t seeds[kOctMax])
-    {
-        const int lane = threadIdx.x & 31;
-        unsigned pend = __ballot_sync(FULL, count > 0);
-        while (pend) {
-            const bool mine = (pend >> lane) & 1u;
-            int incl = mine ? count : 0;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const int v = __shfl_up_sync(FULL, incl, o);
-                if (lane >= o) incl += v;
-            }
-            // (a lane lists at most 12 cells, so the first that waits always fits)
-            const bool go = mine && incl <= kOctList;
-            const unsigned gm = __ballot_sync(FULL, go);
-            const int total = __shfl_sync(FULL, incl, 31 - __clz(gm));
-            if (go) {
-                uint4 *to = list + (incl - count);
-#pragma unroll
-                for (int o = 0; o < kOctMax; ++o) {
-                    const uint32_t kind = (kinds >> (2 * o)) & 3u;
-                    if (!kind) continue;
-                    const int r = (rot >> (2 * o)) & 3u;
-                    const int s1 = r == 2 ? 0 : r + 1, s2 = r == 0 ? 2 : r - 1;
-                    if (kind & 1u) *to++ = make_uint4((uint32_t)base[o] + 1u, seeds[o], place(threadIdx.x, o, s2), L.n_imp);
-                    if (kind & 2u) *to++ = make_uint4((uint32_t)base[o] - 1u, seeds[o], place(threadIdx.x, o, r), L.n_imp);
-                    if (kind == 3u) *to++ = make_uint4((uint32_t)base[o], seeds[o], place(threadIdx.x, o, s1), L.n_imp);
-                }
-            }
-            __syncwarp();
-            const int k = lane & 7;
-            for (int e = lane >> 3; e < total; e += 4) {
-                const uint4 q = list[e];
-                float v = kNoImpulse;
-                if ((uint32_t)k < q.w) {
-                    const uint32_t s = xxhash2(q.x, q.y) + 1u;
-                    const uint32_t r1 = pcg_draw(sj[2 + 2 * k], s);
-                    const uint32_t r2 = pcg_draw(sj[3 + 2 * k], s);
-                    v = __uint_as_float(__float_as_uint(unit_float(r1)) | (~r2 & 0x80000000u));
-                }
-                cbase[q.z + (k >> 2) * (4 * kOctThreads) + (k & 3)] = v;
-            }
-            __syncwarp();
-            pend &= ~gm;
-        }
     }
 
     __device__ __forceinline__ float value(const LaneField &L, float px, float py, float pz,
@@ -3346,18 +3391,12 @@ struct EvalCoopOct {
             const int ci = (int)fl;
             const bool ok = (valid >> o) & 1u;
             if (act && (!ok || ci != base[o])) {
-                const bool up = ok && ci == base[o] + 1, down = ok && ci == base[o] - 1;
-                int r = (rot >> (2 * o)) & 3u;
-                r = up ? (r == 2 ? 0 : r + 1) : (down ? (r == 0 ? 2 : r - 1) : 0);   // up: the old middle becomes the low cell
-                rot = (rot & ~(3u << (2 * o))) | ((uint32_t)r << (2 * o));
-                base[o] = ci;
+                kinds |= window_turn(o, ci, ok, base[o], rot, count);
                 valid |= 1u << o;
-                kinds |= (up ? 1u : (down ? 2u : 3u)) << (2 * o);
-                count += up || down ? 1 : 3;
             }
         }
         refills += (uint32_t)count;
-        fill(kinds, count, L, seeds);
+        window_fill<kOctMax>(list, cbase, sj, kinds, count, base, rot, seeds, L.n_imp);
         float total = 0.0f;
 #pragma unroll
         for (int o = 0; o < kOctMax; ++o) {
@@ -3369,10 +3408,10 @@ struct EvalCoopOct {
             for (int c = 0; c < 3; ++c) {
                 const float tl = __fsub_rn(frac[o], (float)(c - 1));
                 const int slot = c == 0 ? r : (c == 1 ? (r == 2 ? 0 : r + 1) : (r == 0 ? 2 : r - 1));
-                const float4 *row = reinterpret_cast<const float4 *>(cbase + place(threadIdx.x, o, slot));
+                const float4 *row = reinterpret_cast<const float4 *>(cbase + window_place(threadIdx.x, o, slot));
 #pragma unroll
                 for (int h = 0; h < 2; ++h) {
-                    const float4 q4 = row[h * kOctThreads];
+                    const float4 q4 = row[h * kWinThreads];
                     const float qs[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
@@ -3664,6 +3703,10 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
     constexpr int G = Eval::kGroup;
     const bool lead = G == 1 || (lane & (G - 1)) == 0;
     const uint32_t one = lead ? 1u : 0u;
+    // single lanes pull flights when so many are idle: the pull's dependent loads and set-up
+    // hold the whole warp (4.2 M sphere flights 6.17 ms pulling at once, 6.04 at 2, 5.79 at
+    // 4, 5.66 at 8 and at 12)
+    constexpr int kPull = G == 1 && Eval::kSetup == 4 ? 8 : 1;
     constexpr bool kOwn3D = G > 1 && IsSkip3D<Eval>::value;     // marches on with its own evaluator
     uint32_t *work = a.work + (RESUME ? (CERT ? 1 : 2) : 0);
     const unsigned lt_mask = (1u << (lane & ~(G - 1))) - 1u;
@@ -3720,7 +3763,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
     for (;;) {
         const bool need = phase == PH_IDLE && !drained;
         const unsigned need_mask = __ballot_sync(FULL, need && lead);
-        if (need_mask) {
+        if (__popc(need_mask) >= kPull || (need_mask && !__any_sync(FULL, phase != PH_IDLE))) {
             const int leader = __ffs(need_mask) - 1;
             uint32_t base = 0;
             if (lane == leader) base = atomicAdd(work, (uint32_t)__popc(need_mask));
@@ -3756,6 +3799,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                             near_t = on.w;
                             far_t = df.w;
                             first = st.first;
+                            t_direct = st.direct;
                             step = st.step;
                             t0 = st.t0;
                             curv = st.curv;
@@ -3775,6 +3819,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                                 step = __fdiv_rn(__fsub_rn(far_t, near_t), (float)m.min_step);
                                 if (m.step_size < step) step = m.step_size;
                                 t0 = __fadd_rn(near_t, __fmul_rn(step, fl.jitter));
+                                t_direct = t_direct_ok(t0, step, far_t);
                             }
                         }
                         if (!ok) {
@@ -3786,7 +3831,6 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                             c_invalid += one;
                         } else {
                             max_steps = m.max_steps;
-                            t_direct = t_direct_ok(t0, step, far_t);
                             th = near_t;
                             tl = 0.0f;
                             steps = 0;
@@ -3854,14 +3898,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
         if constexpr (CERT) {
             // every phase on the one evaluator (its value is EvalGeneric's), so that
             // the lanes of a warp never run two
-            if constexpr (G > 1)
-                f = ev.certified(L, p[0], p[1], p[2], id, margin);
-            else
-                f = value_1d_cert(L, p[0], p[1], p[2], id, [&](float z, uint32_t seed, float ls) {
-                    float v, dv;
-                    noise1d_generic<false, true>(*L.m, z, seed, v, dv, ls, &margin);
-                    return v;
-                });
+            f = ev.certified(L, p[0], p[1], p[2], id, margin, live);
             c_refills += 3;
         } else {
             if constexpr (G > 1) {
@@ -4825,16 +4862,17 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
         }, [&] {
             if (!plain) {
                 const void *fn = (const void *)k_march<EvalCoopOct, false>;
-                const size_t smem = smem_oct(std::max<uint32_t>(a.max_oct, a.any_mr ? 2u : 1u));
-                failed = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_oct(kOctMax));
+                const size_t smem = smem_window(std::max<uint32_t>(a.max_oct, a.any_mr ? 2u : 1u));
+                failed = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_window(kOctMax));
                 k_march<EvalCoopOct, false><<<grid(fn, smem), 256, smem, stream>>>(b);
             } else if (a.all_grid) {
-                const void *fn = (const void *)k_march<EvalCoop1D<8, true>, false>;
-                k_march<EvalCoop1D<8, true>, false><<<grid(fn), 256, 0, stream>>>(b);
+                using Grid = EvalCoop1D<8, true, true>;
+                const void *fn = (const void *)k_march<Grid, false>;
+                k_march<Grid, false><<<grid(fn, smem_window(1)), 256, smem_window(1), stream>>>(b);
             } else if (a.fast_window == 0u) {
                 // the impulse window in shared memory (the default)
                 const void *fn = (const void *)k_march<EvalCoop1D<8, false, true>, false>;
-                k_march<EvalCoop1D<8, false, true>, false><<<grid(fn, kSmem1D), 256, kSmem1D, stream>>>(b);
+                k_march<EvalCoop1D<8, false, true>, false><<<grid(fn, smem_window(1)), 256, smem_window(1), stream>>>(b);
             } else {
                 const void *fn = (const void *)k_march<EvalCoop1D<8>, false>;
                 k_march<EvalCoop1D<8>, false><<<grid(fn), 256, 0, stream>>>(b);
@@ -4864,8 +4902,9 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
             const void *fn = (const void *)k_march<EvalGroup1D<true, false>, true, true>;
             k_march<EvalGroup1D<true, false>, true, true><<<grid(fn, 0, false, 8), 256, 0, stream>>>(b);
         }, [&] {
-            const void *fn = (const void *)k_march<EvalGeneric4, true, true>;
-            k_march<EvalGeneric4, true, true><<<grid(fn, 0, false), 256, 0, stream>>>(b);
+            using Cert = EvalCoop1D<8, false, true>;
+            const void *fn = (const void *)k_march<Cert, true, true>;
+            k_march<Cert, true, true><<<grid(fn, smem_window(1), false), 256, smem_window(1), stream>>>(b);
         });
         b.queue_in = 2;
     }
@@ -4875,7 +4914,7 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
         const void *fn = (const void *)k_march<EvalGroup3D<32>, true>;
         k_march<EvalGroup3D<32>, true><<<grid(fn, kSmemG3<32>, false, 32), 256, kSmemG3<32>, stream>>>(b);
     } else if (group1) {
-        sized(true, kFewPrecise, [&] {
+        sized(true, plain ? kFewPrecise : kFewPreciseGeneral, [&] {
             if (plain) {
                 const void *fn = (const void *)k_march<EvalGroup1D<true, false>, true>;
                 k_march<EvalGroup1D<true, false>, true><<<grid(fn, 0, false, 8), 256, 0, stream>>>(b);

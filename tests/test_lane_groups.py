@@ -10,6 +10,7 @@ import pytest
 from gpis_extend_gb300 import abi, runtime, workloads
 from oracle import oracle
 from test_gpu_parity import flights_vs_oracle
+from test_skipping import sphere_grid
 
 pytestmark = pytest.mark.gpu
 
@@ -103,12 +104,16 @@ def test_gpu_1d_fast_passes_agree(kind):
     assert two.n > 45_000 and np.array_equal(whole2[:sec.n].view(np.uint32), parts2.view(np.uint32))
 
 
+def sphere_grid_stationary():
+    return abi.attach_grid(workloads.sphere_medium(), sphere_grid())
+
+
 def torus_stationary(**kw):
     return workloads.torus_plane_medium(nonstationary=False, octaves=1, **kw)
 
 
 @pytest.mark.parametrize("kind,n", [("octaves", 45001), ("multires", 45001), ("nonstationary", 46000), ("sphere", 40001),
-                                    ("torus", 40961), ("plane", 41003)])
+                                    ("torus", 40961), ("plane", 41003), ("grid", 40500)])
 def test_gpu_1d_lane_passes_match_oracle(kind, n):
     """Batches just above the limits of the group fast passes: the cooperative single-lane
     passes, whose evaluations decide steps on both sides (the slope bound of several
@@ -116,6 +121,8 @@ def test_gpu_1d_lane_passes_match_oracle(kind, n):
     reach of stationary media with a sphere, torus and linear mean)."""
     if kind == "torus":
         make, flights, half = torus_stationary, workloads.torus_flights, 2.0
+    elif kind == "grid":
+        make, flights, half = sphere_grid_stationary, workloads.sphere_flights, 1.5
     elif kind == "plane":
         make = lambda: workloads.sphere_medium(mean_kind=abi.MEAN_PLANE, mean_params=(0.0, 0.8, 0.6, 0.1))
         flights, half = workloads.sphere_flights, 1.5
