@@ -1967,8 +1967,65 @@ __device__ __forceinline__ float cond3d_value_precise(const DevMedium &m, const 
     return __fadd_rn(__fmul_rn(f, co.vs), gv);
 }
 
-// The precise value of a 1D medium; noise(j, z, seed, ls) gives the normalized noise of
-// octave or level j at the coordinate z (noise1d_precise, or a lane group's share of it).
+// The precise noise of one octave or level of a 1D medium with its conditioning splats;
+// noise_at(j, z, seed, ls) gives the normalized noise at the coordinate z (noise1d_precise,
+// or a lane group's share of it).  den2: 2 (a sqrt2)^2 at the local scale a
+// (covarianceKernel1DVal / 1stGrad, GPFunctions.cpp:850-862).
+__device__ __forceinline__ float precise_den2(const DevMedium &m, const LaneField &L, float ls)
+{
+    const float a = splat_cov_1d(ls, L.ls_o);
+    if (a == 1.0f) return m.cov_den2;
+    const float s2 = (float)((double)a * 1.4142135623730951);
+    return (float)(2.0 * (double)__fmul_rn(s2, s2));
+}
+
+__device__ __forceinline__ void precise_kernels(float d, float den2, float &k0, float &k1)
+{
+    k0 = cr_expf(-__fdiv_rn(__fmul_rn(d, d), den2));
+    // (float)(-2 d / den2 * k0) with the quotient and product carried in float-float: the
+    // double expression's rounding without FP64 division
+    const float r = -2.0f * d;
+    const float qh = __fdiv_rn(r, den2);
+    const float ql = __fdiv_rn(__fmaf_rn(-qh, den2, r), den2);
+    const float ph = __fmul_rn(qh, k0);
+    k1 = __fadd_rn(ph, __fmaf_rn(ql, k0, __fmaf_rn(qh, k0, -ph)));
+}
+
+template <class Noise>
+__device__ __forceinline__ float precise_octave(const LaneField &L, float px, float py, float pz, int k, float ls,
+                                                float den2, float vs, float gz, float oz, Noise noise_at)
+{
+    const DevMedium &m = *L.m;
+    const float z = m.n_oct == 1 && m.ls_kind == 0u ? ray_coord(L.li, L.n, px, py, pz)
+                                                      : ray_coord_oct(m, L.n, px, py, pz, oct_scale(m, k));
+    float noise = noise_at(k, z, L.seed + oct_seed(m, k), ls);
+    if (L.cond) {
+        float k0, k1;
+        precise_kernels(__fsub_rn(z, oz), den2, k0, k1);
+        noise = __fadd_rn(noise, __fmul_rn(1.0f, __fadd_rn(__fmul_rn(vs, k0), __fmul_rn(gz, k1))));
+    }
+    return noise;
+}
+
+template <class Noise>
+__device__ __forceinline__ float precise_level(const LaneField &L, float px, float py, float pz, int j, const MrLevels &lv,
+                                               Noise noise_at)
+{
+    const DevMedium &m = *L.m;
+    const float s = j ? lv.s[1] : lv.s[0];
+    const float z = ray_coord_oct(m, L.n, px, py, pz, s);
+    float noise = noise_at(j, z, L.seed + (j ? lv.seed[1] : lv.seed[0]), 1.0f);
+    if (L.cond) {
+        const float oz = ray_coord_oct(m, L.n, L.o[0], L.o[1], L.o[2], s);
+        float k0, k1;
+        precise_kernels(__fsub_rn(z, oz), m.cov_den2, k0, k1);
+        const float vs0 = __fmul_rn(L.vs, k0), gz0 = __fmul_rn(__fmul_rn(s, L.gsz), k1);
+        noise = __fadd_rn(noise, __fmul_rn(j ? L.mr_ow[1] : L.mr_ow[0], __fadd_rn(vs0, gz0)));
+    }
+    return noise;
+}
+
+// The precise value of a 1D medium.
 template <class Noise>
 __device__ __forceinline__ float field_precise_1d(const LaneField &L, float px, float py, float pz, int &id, Noise noise_at)
 {
@@ -1978,59 +2035,17 @@ __device__ __forceinline__ float field_precise_1d(const LaneField &L, float px, 
         const MrLevels lv = mr_levels(m, ls_value_precise(m, px, pz));
         float nl[2];
 #pragma unroll 1
-        for (int j = 0; j < 2; ++j) {
-            const float z = ray_coord_oct(m, L.n, px, py, pz, lv.s[j]);
-            float noise = noise_at(j, z, L.seed + lv.seed[j], 1.0f);
-            if (L.cond) {
-                const float oz = ray_coord_oct(m, L.n, L.o[0], L.o[1], L.o[2], lv.s[j]);
-                const float d = __fsub_rn(z, oz);
-                const float den2 = m.cov_den2;
-                const float k0 = cr_expf(-__fdiv_rn(__fmul_rn(d, d), den2));
-                const float r = -2.0f * d;
-                const float qh = __fdiv_rn(r, den2);
-                const float ql = __fdiv_rn(__fmaf_rn(-qh, den2, r), den2);
-                const float ph = __fmul_rn(qh, k0);
-                const float k1 = __fadd_rn(ph, __fmaf_rn(ql, k0, __fmaf_rn(qh, k0, -ph)));
-                const float vs0 = __fmul_rn(L.vs, k0);
-                const float gz0 = __fmul_rn(__fmul_rn(lv.s[j], L.gsz), k1);
-                noise = __fadd_rn(noise, __fmul_rn(L.mr_ow[j], __fadd_rn(vs0, gz0)));
-            }
-            nl[j] = noise;
-        }
+        for (int j = 0; j < 2; ++j) nl[j] = precise_level(L, px, py, pz, j, lv, noise_at);
         const float nb = __fadd_rn(__fmul_rn(lv.w[0], nl[0]), __fmul_rn(lv.w[1], nl[1]));
         return mean_plus_precise(m, __fmul_rn(L.sigma, nb), px, py, pz, id);
     }
     const float ls = ns_scale_precise(m, px, pz);
+    const float den2 = L.cond ? precise_den2(m, L, ls) : 0.0f;
     float an = 0.0f;
     for (int k = 0; k < (int)m.n_oct; ++k) {
-        const float sc = oct_scale(m, k);
-        const float z = m.n_oct == 1 && m.ls_kind == 0u ? ray_coord(L.li, L.n, px, py, pz)
-                                                          : ray_coord_oct(m, L.n, px, py, pz, sc);
-        float noise = noise_at(k, z, L.seed + oct_seed(m, k), ls);
-        if (L.cond) {
-            // covarianceKernel1DVal / 1stGrad (GPFunctions.cpp:850-862) at the local
-            // scale a: den2 = 2 (a sqrt2)^2 in float, the derivative in double
-            float vs, gz, oz;
-            lane_cond_1d(L, k, vs, gz, oz);
-            const float a = splat_cov_1d(ls, L.ls_o);
-            float den2 = m.cov_den2;
-            if (a != 1.0f) {
-                const float s2 = (float)((double)a * 1.4142135623730951);
-                den2 = (float)(2.0 * (double)__fmul_rn(s2, s2));
-            }
-            const float d = __fsub_rn(z, oz);
-            const float k0 = cr_expf(-__fdiv_rn(__fmul_rn(d, d), den2));
-            // (float)(-2 d / den2 * k0) with the quotient and product carried in
-            // float-float: the double expression's rounding without FP64 division
-            const float r = -2.0f * d;
-            const float qh = __fdiv_rn(r, den2);
-            const float ql = __fdiv_rn(__fmaf_rn(-qh, den2, r), den2);
-            const float ph = __fmul_rn(qh, k0);
-            const float k1 = __fadd_rn(ph, __fmaf_rn(ql, k0, __fmaf_rn(qh, k0, -ph)));
-            const float vs0 = __fmul_rn(vs, k0);
-            const float gz0 = __fmul_rn(gz, k1);
-            noise = __fadd_rn(noise, __fmul_rn(1.0f, __fadd_rn(vs0, gz0)));
-        }
+        float vs = 0.0f, gz = 0.0f, oz = 0.0f;
+        if (L.cond) lane_cond_1d(L, k, vs, gz, oz);
+        const float noise = precise_octave(L, px, py, pz, k, ls, den2, vs, gz, oz, noise_at);
         an = m.n_oct == 1 ? __fmul_rn(L.sigma, noise) : __fadd_rn(an, __fmul_rn(oct_sigma(m, k), noise));
     }
     return mean_plus_precise(m, an, px, py, pz, id);
@@ -2059,45 +2074,55 @@ __device__ float field_precise(const LaneField &L, float px, float py, float pz,
 }
 
 // ---- fast evaluators ----------------------------------------------------------
-// The fast value of a 1D medium; noise_at(j, z, seed, ls) gives the raw sum of octave or
-// level j at the coordinate z.
-// ls_at: the local scale at the point, as oct_skip_count takes it.
+// The fast value of a 1D medium as the resume passes take it, term by term;
+// noise_at(j, z, seed, ls) gives the raw sum of octave or level j at the coordinate z.
 template <class Noise>
-__device__ __forceinline__ float value_1d(const LaneField &L, float px, float py, float pz, int &id, float &ls_at,
-                                          Noise noise_at)
+__device__ __forceinline__ float value_octave(const LaneField &L, float px, float py, float pz, int k, float ls, float vs,
+                                              float gz, float oz, Noise noise_at)
+{
+    const DevMedium &m = *L.m;
+    const float z = ray_coord_oct(m, L.n, px, py, pz, oct_scale(m, k));
+    float nk = __fmul_rn(noise_at(k, z, L.seed + oct_seed(m, k), ls), inv_norm_1d(m, ls));
+    if (L.cond) {
+        const Cov1D c = cov1d(__fsub_rn(z, oz), splat_cov_1d(ls, L.ls_o));
+        nk = __fadd_rn(nk, __fmaf_rn(vs, c.k0, __fmul_rn(gz, c.k1)));
+    }
+    return nk;
+}
+
+template <class Noise>
+__device__ __forceinline__ float value_level(const LaneField &L, float px, float py, float pz, int j, const MrLevels &lv,
+                                             Noise noise_at)
+{
+    const DevMedium &m = *L.m;
+    const float s = j ? lv.s[1] : lv.s[0];
+    const float z = ray_coord_oct(m, L.n, px, py, pz, s);
+    float nk = __fmul_rn(noise_at(j, z, L.seed + (j ? lv.seed[1] : lv.seed[0]), 1.0f), m.inv_norm1d);
+    if (L.cond) {
+        const Cov1D c = cov1d(__fsub_rn(z, __fdividef(L.ozc, s)));
+        nk = __fmaf_rn(j ? L.mr_ow[1] : L.mr_ow[0], __fmaf_rn(L.vs, c.k0, __fmul_rn(__fmul_rn(s, L.gsz), c.k1)), nk);
+    }
+    return nk;
+}
+
+template <class Noise>
+__device__ __forceinline__ float value_1d(const LaneField &L, float px, float py, float pz, int &id, Noise noise_at)
 {
     const DevMedium &m = *L.m;
     float noise = 0.0f;
     if (m.flags & MF_MULTIRES) {
-        ls_at = ls_value(m, px, pz);
-        const MrLevels lv = mr_levels<true>(m, ls_at);
+        const MrLevels lv = mr_levels<true>(m, ls_value(m, px, pz));
 #pragma unroll 1
-        for (int j = 0; j < 2; ++j) {
-            const float z = ray_coord_oct(m, L.n, px, py, pz, lv.s[j]);
-            float nk = noise_at(j, z, L.seed + lv.seed[j], 1.0f) * m.inv_norm1d;
-            if (L.cond) {
-                const Cov1D c = cov1d(z - __fdividef(L.ozc, lv.s[j]));
-                nk += L.mr_ow[j] * (L.vs * c.k0 + (lv.s[j] * L.gsz) * c.k1);
-            }
-            noise += lv.w[j] * nk;
-        }
-        return L.sigma * noise + lane_mean(L, px, py, pz, id);
+        for (int j = 0; j < 2; ++j) noise = __fmaf_rn(j ? lv.w[1] : lv.w[0], value_level(L, px, py, pz, j, lv, noise_at), noise);
+        return __fmaf_rn(L.sigma, noise, lane_mean(L, px, py, pz, id));
     }
     const float ls = ns_scale(m, px, pz);
-    ls_at = ls;
     for (int k = 0; k < (int)m.n_oct; ++k) {
-        const float sc = oct_scale(m, k);
-        const float z = ray_coord_oct(m, L.n, px, py, pz, sc);
-        float nk = noise_at(k, z, L.seed + oct_seed(m, k), ls) * inv_norm_1d(m, ls);
-        if (L.cond) {
-            float vs, gz, oz;
-            lane_cond_1d(L, k, vs, gz, oz);
-            const Cov1D c = cov1d(z - oz, splat_cov_1d(ls, L.ls_o));
-            nk += vs * c.k0 + gz * c.k1;
-        }
-        noise += oct_sigma(m, k) * nk;
+        float vs = 0.0f, gz = 0.0f, oz = 0.0f;
+        if (L.cond) lane_cond_1d(L, k, vs, gz, oz);
+        noise = __fmaf_rn(oct_sigma(m, k), value_octave(L, px, py, pz, k, ls, vs, gz, oz, noise_at), noise);
     }
-    return noise + lane_mean(L, px, py, pz, id);
+    return __fadd_rn(noise, lane_mean(L, px, py, pz, id));
 }
 
 // Generic evaluator: recomputes every impulse (any impulse count, 1D or 3D).
@@ -2115,8 +2140,7 @@ struct EvalGeneric {
         const DevMedium &m = *L.m;
         float noise;
         if (m.flags & MF_ONE_D) {
-            float ls_at;
-            return value_1d(L, px, py, pz, id, ls_at, [&](int, float z, uint32_t seed, float ls) {
+            return value_1d(L, px, py, pz, id, [&](int, float z, uint32_t seed, float ls) {
                 float v, dv;
                 noise1d_generic<false>(m, z, seed, v, dv, ls);
                 refills += 3;
@@ -2734,12 +2758,16 @@ __device__ __forceinline__ FastPoint fast_point(const LaneField &L, float px, fl
     return q;
 }
 
+// (by selection: the octave may differ between the lanes)
+template <class T>
+__device__ __forceinline__ T pick2(const T (&v)[2], int o) { return o & 1 ? v[1] : v[0]; }
+
 // each octave divides the position by its length multiplier, a multiply when that is a
 // power of two (the same rounding as ray_coord_oct's division)
 __device__ __forceinline__ float fast_coord(const LaneField &L, const FastPoint &q, int o)
 {
     const DevMedium &m = *L.m;
-    const float sc = q.mr ? q.lv.s[o & 1] : oct_scale(m, o);
+    const float sc = q.mr ? pick2(q.lv.s, o) : oct_scale(m, o);
     float x = q.bx, y = q.by, z = q.bz;
     if (sc != 1.0f) {
         if (!q.mr && ((m.oct_pow2 >> o) & 1u)) {
@@ -2754,24 +2782,31 @@ __device__ __forceinline__ float fast_coord(const LaneField &L, const FastPoint 
 
 __device__ __forceinline__ uint32_t fast_seed(const LaneField &L, const FastPoint &q, int o)
 {
-    return L.seed + (q.mr ? q.lv.seed[o & 1] : oct_seed(*L.m, o));
+    return L.seed + (q.mr ? pick2(q.lv.seed, o) : oct_seed(*L.m, o));
 }
 
-__device__ __forceinline__ float fast_share(const LaneField &L, const FastPoint &q, int o, float z, float raw)
+__device__ __forceinline__ float fast_share(const LaneField &L, const FastPoint &q, int o, float z, float raw, float vs,
+                                            float gz, float oz)
 {
     float nk = __fmul_rn(raw, q.inv_norm);
     if (L.cond) {
-        float vs, gz, oz, ow = 1.0f;
-        lane_cond_1d(L, o, vs, gz, oz);
+        float ow = 1.0f;
         if (q.mr) {
-            ow = L.mr_ow[o & 1];
-            oz = __fdividef(oz, q.lv.s[o & 1]);
-            gz = __fmul_rn(gz, q.lv.s[o & 1]);
+            ow = pick2(L.mr_ow, o);
+            oz = __fdividef(oz, pick2(q.lv.s, o));
+            gz = __fmul_rn(gz, pick2(q.lv.s, o));
         }
         const Cov1D kc = cov1d(__fsub_rn(z, oz), q.ca);
         nk = __fmaf_rn(ow, __fmaf_rn(vs, kc.k0, __fmul_rn(gz, kc.k1)), nk);
     }
-    return __fmul_rn(q.mr ? __fmul_rn(L.sigma, q.lv.w[o & 1]) : (L.m->n_oct == 1 ? L.sigma : oct_sigma(*L.m, o)), nk);
+    return __fmul_rn(q.mr ? __fmul_rn(L.sigma, pick2(q.lv.w, o)) : (L.m->n_oct == 1 ? L.sigma : oct_sigma(*L.m, o)), nk);
+}
+
+__device__ __forceinline__ float fast_share(const LaneField &L, const FastPoint &q, int o, float z, float raw)
+{
+    float vs = 0.0f, gz = 0.0f, oz = 0.0f;
+    if (L.cond) lane_cond_1d(L, o, vs, gz, oz);
+    return fast_share(L, q, o, z, raw, vs, gz, oz);
 }
 
 // 1D media of at most 8 impulses per cell: eight lanes per flight, lane k holding impulse
@@ -2879,6 +2914,41 @@ struct EvalGroup1D {
         __syncwarp(mask);
     }
 
+    // the 24 shared terms one after the other
+    __device__ __forceinline__ float row_sum() const
+    {
+        float sv = 0.0f;
+#pragma unroll
+        for (int q = 0; q < 6; ++q) {
+            const float4 t = terms[q];
+            sv = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sv, t.x), t.y), t.z), t.w);
+        }
+        return sv;
+    }
+
+    // raw_sum of window 0 at the local scale ls
+    __device__ __forceinline__ float raw_sum_scaled(const DevMedium &m, float z, uint32_t seed, float ls)
+    {
+        const float tg = __fdiv_rn(z, m.kr_iso);
+        const float fl = floorf(tg);
+        scale_terms(0, (int)fl, __fsub_rn(tg, fl), seed, m.n_imp, __fmul_rn(m.kexp1d, 1.0f / (ls * ls)));
+        return row_sum();
+    }
+
+    // the terms of window o around cell ci, shared
+    __device__ __forceinline__ void scale_terms(int o, int ci, float frac, uint32_t seed, uint32_t n_imp, float kexp)
+    {
+        float c[3], e[3];
+        window(o, ci, seed, n_imp, c);
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+            const float tp = __fsub_rn(__fsub_rn(frac, (float)(d - 1)), fabsf(c[d]));
+            const float x = ex2_approx(kexp * (tp * tp));
+            e[d] = fabsf(tp) < 1.0f ? __uint_as_float(__float_as_uint(x) | (__float_as_uint(c[d]) & 0x80000000u)) : 0.0f;
+        }
+        share(e);
+    }
+
     // the 24 shared terms as the cooperative evaluators add them: even and odd impulses
     __device__ __forceinline__ float pair_sum() const
     {
@@ -2904,7 +2974,7 @@ struct EvalGroup1D {
         float c[3];
         window(j, (int)fl, seed, m.n_imp, c);
         const float il2 = STAT ? 1.0f : 1.0f / (ls * ls);
-        const float kexp = m.kexp1d * il2;
+        const float kexp = __fmul_rn(m.kexp1d, il2);
         float mg = fminf(frac, 1.0f - frac), e[3], dsum = 0.0f;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
@@ -2917,12 +2987,7 @@ struct EvalGroup1D {
         if (der) *der = group_sum<8>(dsum, mask);
         share(e);
         if (FAST) return pair_sum();
-        float sv = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 6; ++q) {
-            const float4 t = terms[q];
-            sv = __fadd_rn(__fadd_rn(__fadd_rn(__fadd_rn(sv, t.x), t.y), t.z), t.w);
-        }
+        const float sv = row_sum();
         if (MARGIN) {
 #pragma unroll
             for (int o = 4; o > 0; o >>= 1) mg = fminf(mg, __shfl_xor_sync(mask, mg, o));
@@ -2963,7 +3028,7 @@ struct EvalGroup1D {
             }
             return total + lane_mean(L, px, py, pz, id);
         } else {
-            return value_1d(L, px, py, pz, id, last_ls, [&](int j, float z, uint32_t seed, float ls) {
+            return value_1d(L, px, py, pz, id, [&](int j, float z, uint32_t seed, float ls) {
                 refills += 3;
                 return raw_sum<false>(*L.m, j, z, seed, ls, nullptr);
             });
@@ -2975,16 +3040,7 @@ struct EvalGroup1D {
     {
         const float tg = __fdiv_rn(z, L.kr);
         const float fl = floorf(tg);
-        const float frac = __fsub_rn(tg, fl);
-        float c[3], e[3];
-        window(o, (int)fl, seed, L.n_imp, c);
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const float tp = __fsub_rn(__fsub_rn(frac, (float)(d - 1)), fabsf(c[d]));
-            const float x = ex2_approx(kexp * (tp * tp));
-            e[d] = fabsf(tp) < 1.0f ? __uint_as_float(__float_as_uint(x) | (__float_as_uint(c[d]) & 0x80000000u)) : 0.0f;
-        }
-        share(e);
+        scale_terms(o, (int)fl, __fsub_rn(tg, fl), seed, L.n_imp, kexp);
         return pair_sum();
     }
 
@@ -3037,6 +3093,111 @@ struct EvalGroup1D {
         return field_precise_1d(L, p[0], p[1], p[2], id, [&](int j, float z, uint32_t seed, float ls) {
             return noise_precise(*L.m, j, z, seed, ls);
         });
+    }
+};
+
+// General 1D media, a warp per flight: eight lanes for each of up to four octaves (or the
+// grid's two levels), which are evaluated side by side where EvalGroup1D takes them one
+// after the other.  Values are EvalGroup1D's: each octave's terms by the same functions,
+// added in the octaves' order.  It repeats the point's and the state machine's work in 32
+// lanes instead of eight, so it serves batches whose longest flights decide the time.
+// Fast pass, warps / eights (us a batch): three octaves, 1 000 flights 1 400 / 2 379, 10 000
+// 2 328 / 2 999, 20 000 3 355 / 3 483, 40 000 5 800 / 4 732; multi-resolution, 3 000 1 439 /
+// 1 949, 10 000 2 207 / 2 198, 30 000 4 774 / 3 658.  Precise pass: three octaves, 10 000
+// 2 863 / 2 999, 100 000 5 416 / 5 676, 300 007 10 229 / 9 489.
+constexpr uint32_t kFewWarps = 12000, kFewWarpsPrecise = 60000;
+template <bool FAST>
+struct EvalWarp1D {
+    static constexpr bool kCollective = false;
+    static constexpr int kGroup = 32;
+    static constexpr int kMinBlocks = 2;
+    static constexpr int kSetup = 8;
+    static constexpr bool kSkip = false;
+    EvalGroup1D<true, FAST> part;       // the octave's eight lanes: one window
+    float last_ls;
+    int o;
+
+    __device__ __forceinline__ void reset() { part.reset(); last_ls = 1.0f; }
+    __device__ __forceinline__ void bind(const PcgJump *t)
+    {
+        part.bind(t);
+        o = (threadIdx.x & 31) >> 3;
+    }
+    // octave i's coefficients for the lanes of octave i
+    static __device__ __forceinline__ void own(const LaneField &L, int i, float &vs, float &gz, float &oz)
+    {
+        vs = L.vs;
+        gz = L.gsz;
+        oz = L.ozc;
+#pragma unroll
+        for (int k = 1; k < 4; ++k)
+            if (i == k) {
+                vs = L.c3.oct[k].vs;
+                gz = L.c3.oct[k].gs[2];
+                oz = L.c3.oct[k].gs[0];
+            }
+    }
+    __device__ __forceinline__ int octave(const DevMedium &m) const
+    {
+        return min(o, (m.flags & MF_MULTIRES) ? 1 : (int)m.n_oct - 1);
+    }
+
+    __device__ __forceinline__ float value(const LaneField &L, float px, float py, float pz, int &id, uint32_t &refills,
+                                           bool)
+    {
+        const DevMedium &m = *L.m;
+        const int i = octave(m);
+        float vs, gz, oz;
+        refills += 3;
+        if constexpr (FAST) {
+            const FastPoint q = fast_point(L, px, py, pz);
+            last_ls = q.ls;
+            own(L, q.mr ? 0 : i, vs, gz, oz);
+            const float z = fast_coord(L, q, i);
+            const float share = fast_share(L, q, i, z, part.octave_sum(L, 0, z, fast_seed(L, q, i), q.kexp), vs, gz, oz);
+            float total = 0.0f;
+            const int n = q.mr ? 2 : (int)m.n_oct;
+            for (int k = 0; k < n; ++k) total = __fadd_rn(total, __shfl_sync(FULL, share, 8 * k));
+            return total + lane_mean(L, px, py, pz, id);
+        } else {
+            auto raw = [&](int, float z, uint32_t seed, float ls) {
+                return part.raw_sum_scaled(m, z, seed, ls);
+            };
+            float noise = 0.0f;
+            if (m.flags & MF_MULTIRES) {
+                const MrLevels lv = mr_levels<true>(m, ls_value(m, px, pz));
+                const float nk = value_level(L, px, py, pz, i, lv, raw);
+                for (int k = 0; k < 2; ++k) noise = __fmaf_rn(k ? lv.w[1] : lv.w[0], __shfl_sync(FULL, nk, 8 * k), noise);
+                return __fmaf_rn(L.sigma, noise, lane_mean(L, px, py, pz, id));
+            }
+            own(L, i, vs, gz, oz);
+            const float nk = value_octave(L, px, py, pz, i, ns_scale(m, px, pz), vs, gz, oz, raw);
+            for (int k = 0; k < (int)m.n_oct; ++k) noise = __fmaf_rn(oct_sigma(m, k), __shfl_sync(FULL, nk, 8 * k), noise);
+            return __fadd_rn(noise, lane_mean(L, px, py, pz, id));
+        }
+    }
+
+    __device__ __forceinline__ float precise(const LaneField &L, const float p[3], int &id)
+    {
+        const DevMedium &m = *L.m;
+        const int i = octave(m);
+        auto noise_at = [&](int, float z, uint32_t seed, float ls) { return part.noise_precise(m, 0, z, seed, ls); };
+        if (m.flags & MF_MULTIRES) {
+            const MrLevels lv = mr_levels(m, ls_value_precise(m, p[0], p[2]));
+            const float n = precise_level(L, p[0], p[1], p[2], i, lv, noise_at);
+            const float nb = __fadd_rn(__fmul_rn(lv.w[0], __shfl_sync(FULL, n, 0)), __fmul_rn(lv.w[1], __shfl_sync(FULL, n, 8)));
+            return mean_plus_precise(m, __fmul_rn(L.sigma, nb), p[0], p[1], p[2], id);
+        }
+        const float ls = ns_scale_precise(m, p[0], p[2]);
+        float vs, gz, oz;
+        own(L, i, vs, gz, oz);
+        const float n = precise_octave(L, p[0], p[1], p[2], i, ls, L.cond ? precise_den2(m, L, ls) : 0.0f, vs, gz, oz, noise_at);
+        float an = 0.0f;
+        for (int k = 0; k < (int)m.n_oct; ++k) {
+            const float nk = __shfl_sync(FULL, n, 8 * k);
+            an = m.n_oct == 1 ? __fmul_rn(L.sigma, nk) : __fadd_rn(an, __fmul_rn(oct_sigma(m, k), nk));
+        }
+        return mean_plus_precise(m, an, p[0], p[1], p[2], id);
     }
 };
 
@@ -3585,6 +3746,7 @@ __device__ __forceinline__ float skip_scale(const DevMedium &m, float px, float 
 // the evaluators whose fast pass skips by oct_skip_count, and the cap of each
 template <class E> struct IsOct { static constexpr bool value = false; static constexpr int cap = 0; };
 template <> struct IsOct<EvalCoopOct> { static constexpr bool value = true; static constexpr int cap = 16; };
+template <> struct IsOct<EvalWarp1D<true>> { static constexpr bool value = true; static constexpr int cap = 16; };
 template <> struct IsOct<EvalGroup1D<false, true>> { static constexpr bool value = true; static constexpr int cap = 16; };
 
 template <class E> struct IsSkip3D { static constexpr bool value = false; };
@@ -3755,7 +3917,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
     const int q_in = RESUME && a.queue ? a.queue_in : 0;
     const uint32_t *queue_in = q_in ? a.queue + (size_t)(q_in - 1) * a.n : nullptr;
     const uint32_t n_live = q_in ? a.work[kWorkQueueLen + q_in - 1] : live_n(a);
-    if (n_live < a.run_lo || n_live >= a.run_hi) return;
+    if (n_live == 0u || n_live < a.run_lo || n_live >= a.run_hi) return;
     // the queue this pass hands its saved flights on to
     uint32_t *queue_out = a.queue ? a.queue + (CERT ? (size_t)a.n : 0) : nullptr;
     uint32_t *queue_len = a.work + kWorkQueueLen + (CERT ? 1 : 0);
@@ -4246,15 +4408,12 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
     const unsigned long long s0 = warp_sum(c_flights), s1 = warp_sum(c_steps), s2 = warp_sum(c_refine),
                              s3 = warp_sum(c_hits), s4 = warp_sum(c_limit), s5 = warp_sum(c_invalid),
                              s6 = warp_sum(c_refills), s7 = warp_sum(c_skipped);
-    if (lane == 0 && a.counters) {
-        atomicAdd(a.counters + 0, s0);
-        atomicAdd(a.counters + 1, s1);
-        atomicAdd(a.counters + 2, s2);
-        atomicAdd(a.counters + 3, s3);
-        atomicAdd(a.counters + 4, s4);
-        atomicAdd(a.counters + 5, s5);
-        atomicAdd(a.counters + 6, s6);
-        atomicAdd(a.counters + 7, s7);
+    // (only what there is to add: 2 432 warps adding eight zeros held an idle pass 16 us)
+    const unsigned long long sums[8] = {s0, s1, s2, s3, s4, s5, s6, s7};
+    if (a.counters && lane == 0) {
+#pragma unroll
+        for (int k = 0; k < 8; ++k)
+            if (sums[k]) atomicAdd(a.counters + k, sums[k]);
     }
 }
 
@@ -4849,6 +5008,15 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
         b.run_lo = 0;
         b.run_hi = all;
     };
+    // the lane groups of general media below `few` flights: a warp per flight
+    auto by_octaves = [&](uint32_t few, auto warps, auto groups, bool device_count) {
+        const uint32_t hi = b.run_hi;
+        b.run_hi = std::min(few, hi);
+        if (device_count || a.n < few) warps();
+        b.run_lo = few;
+        b.run_hi = hi;
+        if (a.n >= few) groups();
+    };
     if (group1) {
         cudaError_t failed = cudaSuccess;
         sized(a.n_dev != nullptr, plain ? kFewPlain : kFewGeneral, [&] {
@@ -4856,8 +5024,13 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
                 const void *fn = (const void *)k_march<EvalGroup1D<true, true>, false>;
                 k_march<EvalGroup1D<true, true>, false><<<grid(fn, 0, true, 8), 256, 0, stream>>>(b);
             } else {
-                const void *fn = (const void *)k_march<EvalGroup1D<false, true>, false>;
-                k_march<EvalGroup1D<false, true>, false><<<grid(fn, 0, true, 8), 256, 0, stream>>>(b);
+                by_octaves(kFewWarps, [&] {
+                    const void *fn = (const void *)k_march<EvalWarp1D<true>, false>;
+                    k_march<EvalWarp1D<true>, false><<<grid(fn, 0, true, 32), 256, 0, stream>>>(b);
+                }, [&] {
+                    const void *fn = (const void *)k_march<EvalGroup1D<false, true>, false>;
+                    k_march<EvalGroup1D<false, true>, false><<<grid(fn, 0, true, 8), 256, 0, stream>>>(b);
+                }, a.n_dev != nullptr);
             }
         }, [&] {
             if (!plain) {
@@ -4919,8 +5092,13 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
                 const void *fn = (const void *)k_march<EvalGroup1D<true, false>, true>;
                 k_march<EvalGroup1D<true, false>, true><<<grid(fn, 0, false, 8), 256, 0, stream>>>(b);
             } else {
-                const void *fn = (const void *)k_march<EvalGroup1D<false, false>, true>;
-                k_march<EvalGroup1D<false, false>, true><<<grid(fn, 0, false, 8), 256, 0, stream>>>(b);
+                by_octaves(kFewWarpsPrecise, [&] {
+                    const void *fn = (const void *)k_march<EvalWarp1D<false>, true>;
+                    k_march<EvalWarp1D<false>, true><<<grid(fn, 0, false, 32), 256, 0, stream>>>(b);
+                }, [&] {
+                    const void *fn = (const void *)k_march<EvalGroup1D<false, false>, true>;
+                    k_march<EvalGroup1D<false, false>, true><<<grid(fn, 0, false, 8), 256, 0, stream>>>(b);
+                }, true);
             }
         }, [&] {
             const void *fn = (const void *)k_march<EvalGeneric, true>;

@@ -92,7 +92,9 @@ def test_gpu_1d_fast_passes_agree(kind):
     prim = flights(48_000, desc)
     with runtime.Context(desc) as ctx:
         whole = ctx.trace_host(prim)
+        # 6 000: a warp per flight in media of several octaves, 16 000: eight lanes
         parts = np.concatenate([ctx.trace_host(prim.subset(np.arange(k, k + 6000))) for k in range(0, prim.n, 6000)])
+        eights = np.concatenate([ctx.trace_host(prim.subset(np.arange(k, k + 16000))) for k in range(0, prim.n, 16000)])
         sec, _ = workloads.secondary_flights(prim, whole, desc, half=half)
         two = abi.FlightBatch(2 * sec.n)
         for name in ("origin_near", "dir_far", "seeds", "prev"):
@@ -101,6 +103,7 @@ def test_gpu_1d_fast_passes_agree(kind):
         parts2 = np.concatenate([ctx.trace_host(sec.subset(np.arange(k, min(k + 6000, sec.n))))
                                  for k in range(0, sec.n, 6000)])
     assert np.array_equal(whole.view(np.uint32), parts.view(np.uint32))
+    assert np.array_equal(whole.view(np.uint32), eights.view(np.uint32))
     assert two.n > 45_000 and np.array_equal(whole2[:sec.n].view(np.uint32), parts2.view(np.uint32))
 
 
