@@ -265,6 +265,9 @@ struct gpis_ctx {
     uint32_t *d_work = nullptr;
     unsigned long long *d_counters = nullptr;
     size_t cap = 0;
+    // the renderer's buffers, kept between renders while they are small (render_block)
+    void *d_render = nullptr;
+    size_t render_cap = 0;
     // staging of the host entry point
     char *d_stage = nullptr;
     size_t stage_cap = 0;
@@ -298,6 +301,7 @@ void release(gpis_ctx *c)
     cudaFree(c->d_work);
     cudaFree(c->d_counters);
     cudaFree(c->d_stage);
+    cudaFree(c->d_render);
     for (cudaEvent_t e : c->ev_pool) cudaEventDestroy(e);
     for (cudaEvent_t e : c->ev_pending) cudaEventDestroy(e);
     if (c->stream) cudaStreamDestroy(c->stream);
@@ -661,6 +665,34 @@ int gpis_tune_get(gpis_ctx *ctx, uint32_t key, uint64_t *value)
     if (key > GPIS_TUNE_PRECISE_DECISIONS) return fail(GPIS_EINVAL, "unknown schedule knob");
     *value = ctx->tune[key];
     return GPIS_OK;
+}
+
+// The renderer's block of at least `bytes`.  A render allocated and freed 25 buffers, about
+// a millisecond of a small image's time; a block of up to 256 MiB (a pass of 400 000 paths)
+// now stays with the context, a larger one, whose render takes far longer, is given back by
+// gpis_internal_render_done.
+constexpr size_t kRenderKeep = (size_t)256 << 20;
+
+__attribute__((visibility("hidden"))) int gpis_internal_render_block(gpis_ctx *ctx, size_t bytes, void **block)
+{
+    if (!ctx || !block) return fail(GPIS_EINVAL, "null argument");
+    if (bytes > ctx->render_cap) {
+        cudaFree(ctx->d_render);
+        ctx->d_render = nullptr;
+        ctx->render_cap = 0;
+        CUDA_TRY(cudaMalloc(&ctx->d_render, bytes), "allocate render buffers");
+        ctx->render_cap = bytes;
+    }
+    *block = ctx->d_render;
+    return GPIS_OK;
+}
+
+__attribute__((visibility("hidden"))) void gpis_internal_render_done(gpis_ctx *ctx)
+{
+    if (!ctx || ctx->render_cap <= kRenderKeep) return;
+    cudaFree(ctx->d_render);
+    ctx->d_render = nullptr;
+    ctx->render_cap = 0;
 }
 
 __attribute__((visibility("hidden"))) uint32_t gpis_internal_render_pass(gpis_ctx *ctx)

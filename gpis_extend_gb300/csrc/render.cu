@@ -811,17 +811,16 @@ inline void hcross(const float a[3], const float b[3], float o[3])
     o[2] = a[0] * b[1] - a[1] * b[0];
 }
 
-struct DevBuf {
-    std::vector<void *> ptrs;
-    ~DevBuf() { for (void *p : ptrs) cudaFree(p); }
+// The buffers of one render laid out in one block: a first walk with no base measures it,
+// a second one hands out the places.
+struct Arena {
+    char *base = nullptr;
+    size_t used = 0;
     template <class T>
-    cudaError_t alloc(T *&p, size_t n)
+    void place(T *&p, size_t n)
     {
-        void *v = nullptr;
-        cudaError_t e = cudaMalloc(&v, std::max<size_t>(n, 1) * sizeof(T));
-        if (e == cudaSuccess) ptrs.push_back(v);
-        p = static_cast<T *>(v);
-        return e;
+        p = base ? reinterpret_cast<T *>(base + used) : nullptr;
+        used += (std::max<size_t>(n, 1) * sizeof(T) + 255) & ~(size_t)255;
     }
 };
 
@@ -852,6 +851,8 @@ extern "C" int gpis_internal_nee_live(gpis_ctx *ctx, const gpis_nee_soa *in, flo
                                       const uint32_t *n_dev, void *cuda_stream);
 extern "C" int gpis_internal_ctx_info(gpis_ctx *ctx, int *num_sms, int *profiling, int *prepare_runs);
 extern "C" uint32_t gpis_internal_render_pass(gpis_ctx *ctx);
+extern "C" int gpis_internal_render_block(gpis_ctx *ctx, size_t bytes, void **block);
+extern "C" void gpis_internal_render_done(gpis_ctx *ctx);
 
 namespace {
 
@@ -975,7 +976,6 @@ extern "C" int gpis_render_batch_proposed(gpis_ctx *ctx, gpis_proposal *prop, co
     int num_sms = 1, profiling = 0, prepare_runs = 1;
     gpis_internal_ctx_info(ctx, &num_sms, &profiling, &prepare_runs);
 
-    DevBuf mem;
     RtScene *d_scenes;
     Seg *d_segs;
     PathRec *paths;
@@ -984,53 +984,64 @@ extern "C" int gpis_render_batch_proposed(gpis_ctx *ctx, gpis_proposal *prop, co
     NeeQueue eq{};
     uint32_t *counts, *n_paths;
     unsigned long long *dcnt;
-    RT_TRY(mem.alloc(d_scenes, n_scenes), "allocate scenes");
-    RT_TRY(mem.alloc(d_segs, max_segs), "allocate segments");
-    RT_TRY(mem.alloc(paths, cap), "allocate paths");
-    RT_TRY(mem.alloc(direct, (size_t)cap * 6), "allocate direct light");
-    RT_TRY(mem.alloc(acc, (size_t)total_pixels * 3), "allocate images");
-    RT_TRY(mem.alloc(counts, 3), "allocate queue counters");
-    RT_TRY(mem.alloc(n_paths, 1), "allocate path count");
-    RT_TRY(mem.alloc(dcnt, 5), "allocate counters");
     // the learned arm: features and proposed intervals of the distance queue
     float *feats = nullptr, *ivals = nullptr;
-    if (prop) {
-        RT_TRY(mem.alloc(feats, (size_t)cap * 24), "allocate proposal features");
-        RT_TRY(mem.alloc(ivals, (size_t)cap * 4), "allocate proposal intervals");
-    }
-    for (Queue *qq : {&q, &sq}) {
-        const size_t m = qq == &q ? cap : 2 * (size_t)cap;
-        RT_TRY(mem.alloc(qq->origin_near, m), "allocate queue");
-        RT_TRY(mem.alloc(qq->dir_far, m), "allocate queue");
-        RT_TRY(mem.alloc(qq->prev, m), "allocate queue");
-        RT_TRY(mem.alloc(qq->seeds, m), "allocate queue");
-        RT_TRY(mem.alloc(qq->rec, 2 * m), "allocate queue");
-        RT_TRY(mem.alloc(qq->path, m), "allocate queue");
-        RT_TRY(mem.alloc(qq->payload, m), "allocate queue");
-        RT_TRY(mem.alloc(qq->medium, m), "allocate queue");
-    }
+    auto layout = [&](Arena &mem) {
+        mem.place(d_scenes, n_scenes);
+        mem.place(d_segs, max_segs);
+        mem.place(paths, cap);
+        mem.place(direct, (size_t)cap * 6);
+        mem.place(acc, (size_t)total_pixels * 3);
+        mem.place(counts, 3);
+        mem.place(n_paths, 1);
+        mem.place(dcnt, 5);
+        if (prop) {
+            mem.place(feats, (size_t)cap * 24);
+            mem.place(ivals, (size_t)cap * 4);
+        }
+        for (Queue *qq : {&q, &sq}) {
+            const size_t m = qq == &q ? cap : 2 * (size_t)cap;
+            mem.place(qq->origin_near, m);
+            mem.place(qq->dir_far, m);
+            mem.place(qq->prev, m);
+            mem.place(qq->seeds, m);
+            mem.place(qq->rec, 2 * m);
+            mem.place(qq->path, m);
+            mem.place(qq->payload, m);
+            mem.place(qq->medium, m);
+        }
+        if (any_nee) {
+            // at most two queries per event: the light sample and the MIS phase sample
+            const size_t m = 2 * (size_t)cap;
+            mem.place(eq.origin_near, m);
+            mem.place(eq.dir_far, m);
+            mem.place(eq.prev, m);
+            mem.place(eq.seeds, m);
+            mem.place(eq.point_t, m);
+            mem.place(eq.normal, m);
+            mem.place(eq.out, m);
+            mem.place(eq.a, m);
+            mem.place(eq.b, m);
+            mem.place(eq.c, m);
+            mem.place(eq.path, m);
+            mem.place(eq.medium, m);
+        }
+    };
+    Arena mem;
+    layout(mem);
+    void *block = nullptr;
+    const int brc = gpis_internal_render_block(ctx, mem.used, &block);
+    if (brc) return brc;
+    struct BlockGuard { gpis_ctx *c; ~BlockGuard() { gpis_internal_render_done(c); } } bg{ctx};
+    mem = Arena{static_cast<char *>(block), 0};
+    layout(mem);
     q.count = counts;
     sq.count = counts + 1;
     eq.count = counts + 2;
-    if (any_nee) {
-        // at most two queries per event: the light sample and the MIS phase sample
-        const size_t m = 2 * (size_t)cap;
-        RT_TRY(mem.alloc(eq.origin_near, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.dir_far, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.prev, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.seeds, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.point_t, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.normal, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.out, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.a, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.b, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.c, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.path, m), "allocate NEE queue");
-        RT_TRY(mem.alloc(eq.medium, m), "allocate NEE queue");
-    }
     cudaStream_t st;
     RT_TRY(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking), "create stream");
-    struct StreamGuard { cudaStream_t s; ~StreamGuard() { cudaStreamDestroy(s); } } sg{st};
+    // (the buffers outlive this call: nothing of it may still run when it returns)
+    struct StreamGuard { cudaStream_t s; ~StreamGuard() { cudaStreamSynchronize(s); cudaStreamDestroy(s); } } sg{st};
     cudaEvent_t e0, e1;
     RT_TRY(cudaEventCreate(&e0), "create event");
     RT_TRY(cudaEventCreate(&e1), "create event");
