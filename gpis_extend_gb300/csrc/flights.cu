@@ -87,32 +87,37 @@ __device__ __forceinline__ float ns_scale(const DevMedium &m, float x, float z)
     return __fdiv_rn(q[0] + q[1] * sinf(q[2] * x) * cosf(q[3] * z), m.ls_max);
 }
 
-// The same with the procedural vector evaluated in double, as on Vec3d(p).
-__device__ __forceinline__ float ns_scale_precise(const DevMedium &m, float x, float z)
+// The length scale with the procedural vector evaluated in double, as on Vec3d(p):
+// float-float with a test of the rounding, the double sine and cosine (out of line) for
+// the values it cannot decide.  FP64 runs at 1/64 of the FP32 rate here, and the precise
+// pass of a nonstationary medium waited for it (short_scoreboard 9.7 warps per issue on the
+// multi-resolution grid).
+__device__ __noinline__ float ls_value_double(float a, float b, float fx, float fz, float x, float z)
 {
-    if (m.ls_kind == 0u) return 1.0f;
-    const float *q = m.ls_params;
-    const double v = __dmul_rn(__dmul_rn((double)q[1], sin(__dmul_rn((double)q[2], (double)x))),
-                               cos(__dmul_rn((double)q[3], (double)z)));
-    const float ls = (float)__dadd_rn((double)q[0], v);
-    return __fdiv_rn(ls, m.ls_max);
-}
-
-// ---- multi-resolution grid ---------------------------------------------------------
-// ls(p) of the procedural length scale (the grid's lateral scale): float, and the
-// double evaluation on Vec3d(p) as ns_scale_precise takes it.
-__device__ __forceinline__ float ls_value(const DevMedium &m, float x, float z)
-{
-    const float *q = m.ls_params;
-    return q[0] + q[1] * sinf(q[2] * x) * cosf(q[3] * z);
+    const double v = __dmul_rn(__dmul_rn((double)b, sin(__dmul_rn((double)fx, (double)x))),
+                               cos(__dmul_rn((double)fz, (double)z)));
+    return (float)__dadd_rn((double)a, v);
 }
 
 __device__ __forceinline__ float ls_value_precise(const DevMedium &m, float x, float z)
 {
     const float *q = m.ls_params;
-    const double v = __dmul_rn(__dmul_rn((double)q[1], sin(__dmul_rn((double)q[2], (double)x))),
-                               cos(__dmul_rn((double)q[3], (double)z)));
-    return (float)__dadd_rn((double)q[0], v);
+    float ls;
+    if (ffm_length_scale(q[0], q[1], q[2], q[3], x, z, ls)) return ls;
+    return ls_value_double(q[0], q[1], q[2], q[3], x, z);
+}
+
+__device__ __forceinline__ float ns_scale_precise(const DevMedium &m, float x, float z)
+{
+    return m.ls_kind == 0u ? 1.0f : __fdiv_rn(ls_value_precise(m, x, z), m.ls_max);
+}
+
+// ---- multi-resolution grid ---------------------------------------------------------
+// ls(p) of the procedural length scale (the grid's lateral scale) in float
+__device__ __forceinline__ float ls_value(const DevMedium &m, float x, float z)
+{
+    const float *q = m.ls_params;
+    return q[0] + q[1] * sinf(q[2] * x) * cosf(q[3] * z);
 }
 
 // The two levels around ls: scales, weights and noise-seed offsets
@@ -124,6 +129,14 @@ struct MrLevels {
 };
 
 // FAST: the weights in float (within about 1e-7; the levels are the same).
+__device__ __noinline__ void level_weights_double(float frac, float &w0, float &w1)
+{
+    const double f = (double)frac;
+    const double den = __dsqrt_rn(__dadd_rn(__dsub_rn(1.0, __dmul_rn(2.0, f)), __dmul_rn(__dmul_rn(2.0, f), f)));
+    w0 = (float)__ddiv_rn(__dsub_rn(1.0, f), den);
+    w1 = (float)__ddiv_rn(f, den);
+}
+
 template <bool FAST = false>
 __device__ __forceinline__ MrLevels mr_levels(const DevMedium &m, float ls)
 {
@@ -142,10 +155,7 @@ __device__ __forceinline__ MrLevels mr_levels(const DevMedium &m, float ls)
         r.w[1] = frac * inv;
         return r;
     }
-    const double f = (double)frac;
-    const double den = __dsqrt_rn(__dadd_rn(__dsub_rn(1.0, __dmul_rn(2.0, f)), __dmul_rn(__dmul_rn(2.0, f), f)));
-    r.w[0] = (float)__ddiv_rn(__dsub_rn(1.0, f), den);
-    r.w[1] = (float)__ddiv_rn(f, den);
+    if (!ffm_level_weights(frac, r.w[0], r.w[1])) level_weights_double(frac, r.w[0], r.w[1]);
     return r;
 }
 
