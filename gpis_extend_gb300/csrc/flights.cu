@@ -2837,10 +2837,16 @@ __device__ __forceinline__ float fast_share(const LaneField &L, const FastPoint 
 // (Several octaves since the set-up records: 300 007 flights 9 503 / 10 935, 60 013 on the
 // multi-resolution grid 4 392 / 5 818.)
 constexpr uint32_t kFewCertified = 100000, kFewPrecise = 200000, kFewPreciseGeneral = 1000000;
-// Fast passes the same way: plain media, 509 flights 159 / 253, 20 000 273 / 364, 65 537
-// 484 / 444, 262 144 1 423 / 867; three octaves, 10 000 2 988 / 4 308, 30 000 4 742 / 5 084,
-// 100 000 8 906 / 6 054; multi-resolution, 20 000 2 606 / 3 419, 60 013 5 296 / 4 818.
-constexpr uint32_t kFewPlain = 40000, kFewGeneral = 45000;
+// Fast passes the same way, groups / lanes with their tail on groups: plain media, 10 000
+// flights 251 / 298, 20 000 242 / 268, 40 000 357 / 345, 65 537 425 / 338; three octaves,
+// 20 000 3 281 / 3 174, 40 000 4 443 / 3 488; multi-resolution, 20 000 2 479 / 2 492,
+// 60 013 4 874 / 3 669.
+constexpr uint32_t kFewPlain = 32000, kFewGeneral = 20000;
+// The lanes' tail: the most flights that a warp hands over when none is left to pull, none
+// handed over / 4 / 8 / 16: plain, 65 537 354 / 339 / 338 / 344, 4.2 M 5 518 / 5 507 / 5 502 /
+// 5 532; three octaves, 300 007 9 336 / 8 343 / 9 070 / 9 087; multi-resolution, 60 013 4 172 /
+// 3 669 / 3 858 / 3 801; a grid mean, 500 009 1 415 / 1 444 / 1 462 / 1 485.
+constexpr uint32_t kHandOverPlain = 8, kHandOverGeneral = 4;
 
 // STAT: every medium of the batch is stationary with one octave.  FAST: the fast pass,
 // whose sums keep the cooperative evaluators' order and which takes the slope along; the resume passes' values
@@ -3791,6 +3797,8 @@ constexpr float kPreciseBand = 1e-6f;
 // FlightArgs::work: the passes' fetch counters (fast 0, certified 1, precise 2),
 // then the lengths of the two hand-off queues.
 constexpr int kWorkQueueLen = 3;
+// then the fast pass's tail: the length of its queue and its fetch counter
+constexpr int kWorkTailLen = 5, kWorkTail = 6;
 
 // Appends v to a hand-off queue: one atomic per group of lanes that push together.
 __device__ __forceinline__ void queue_push(uint32_t *q, uint32_t *len, uint32_t v)
@@ -3866,10 +3874,12 @@ __device__ __forceinline__ unsigned long long warp_sum(uint32_t v)
 // saved crossings of the media cert_medium accepts, decides them on fast values
 // where that is certain and hands the rest on (kResumeNoCert) to the precise pass,
 // so that no warp runs both evaluators.
-template <class Eval, bool RESUME, bool CERT = false>
+// TAIL: the fast pass over the flights that a single-lane pass handed over at its end.
+template <class Eval, bool RESUME, bool CERT = false, bool TAIL = false>
 __device__ __forceinline__ void march_flights(const FlightArgs &a)
 {
     static_assert(!CERT || RESUME, "the certified pass is a resume pass");
+    static_assert(!TAIL || !RESUME, "the tail is a fast pass");
     const int lane = threadIdx.x & 31;
     // the first lane of the flight's group fetches, writes and counts for it
     constexpr int G = Eval::kGroup;
@@ -3880,7 +3890,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
     // 4, 5.66 at 8 and at 12)
     constexpr int kPull = G == 1 && Eval::kSetup == 4 ? 8 : 1;
     constexpr bool kOwn3D = G > 1 && IsSkip3D<Eval>::value;     // marches on with its own evaluator
-    uint32_t *work = a.work + (RESUME ? (CERT ? 1 : 2) : 0);
+    uint32_t *work = a.work + (TAIL ? kWorkTail : (RESUME ? (CERT ? 1 : 2) : 0));
     const unsigned lt_mask = (1u << (lane & ~(G - 1))) - 1u;
     // 0.9 and 0.01 as float-float pairs (the reference's double constants)
     const FF kNine = {0.9f, -2.38418579e-08f};
@@ -3919,14 +3929,18 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
     constexpr bool kBothSides = !RESUME && (Eval::kSkip || IsOct<Eval>::value);
     uint32_t ahead = 0, mark_lo = 0xffffffffu, mark_hi = 0;
     int reach = 0;
+    // Once no flight is left to pull, a warp waits for its longest flight with most lanes
+    // idle; its last flights go on in a pass of lane groups, from the same step (the groups'
+    // values are the same bits).
+    constexpr bool kHandsOver = kBothSides && G == 1;
     float prop_a = -INFINITY;   // start of the proposed crossing interval (learned proposal)
     // certified pass: the bound on fac's distance from the reference's (cert_fac)
     float dfac = 0.0f;
     const int prop_cap = a.prop_cap ? (int)a.prop_cap : kMaxSkipProposed;
     // the flights this pass takes: every flight, or the queue the pass before filled
-    const int q_in = RESUME && a.queue ? a.queue_in : 0;
+    const int q_in = TAIL ? 2 : (RESUME && a.queue ? a.queue_in : 0);
     const uint32_t *queue_in = q_in ? a.queue + (size_t)(q_in - 1) * a.n : nullptr;
-    const uint32_t n_live = q_in ? a.work[kWorkQueueLen + q_in - 1] : live_n(a);
+    const uint32_t n_live = TAIL ? a.work[kWorkTailLen] : (q_in ? a.work[kWorkQueueLen + q_in - 1] : live_n(a));
     if (n_live == 0u || n_live < a.run_lo || n_live >= a.run_hi) return;
     // the queue this pass hands its saved flights on to
     uint32_t *queue_out = a.queue ? a.queue + (CERT ? (size_t)a.n : 0) : nullptr;
@@ -3947,13 +3961,13 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                 } else {
                     const uint32_t idx = q_in ? queue_in[item] : item;
                     fid = idx;
-                    if (!RESUME) c_flights += one;
+                    if (!RESUME && !TAIL) c_flights += one;
                     prop_a = (!RESUME && a.proposal) ? a.proposal[idx].x : -INFINITY;
                     bool mok;
                     L.m = medium_of(a, idx, mok);
                     const DevMedium &m = *L.m;
                     uint4 rs = make_uint4(0u, 0u, 0u, 0u);
-                    if (RESUME) rs = a.resume[idx];
+                    if (RESUME || TAIL) rs = a.resume[idx];
                     if (RESUME && (rs.w >> 28) == 0u) {
                         // finished by the fast pass
                     } else if (CERT && ((rs.w >> 28) != (uint32_t)PH_MARCH_P || (rs.w & kResumeNoCert) || !mok ||
@@ -4013,7 +4027,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                             }
                             ev.reset();
                             phase = PH_F0;
-                            if (RESUME) {
+                            if (RESUME || TAIL) {
                                 th = __uint_as_float(rs.x);
                                 tl = __uint_as_float(rs.y);
                                 pf = __uint_as_float(rs.z);
@@ -4025,6 +4039,18 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                         }
                     }
                 }
+            }
+        }
+        if constexpr (kHandsOver) {
+            const unsigned lm = __ballot_sync(FULL, phase != PH_IDLE);
+            if (lm && __popc(lm) <= (int)a.hand_over && __any_sync(FULL, drained)) {
+                if (phase != PH_IDLE) {
+                    if (ahead != 0u) t_after(t0, step, steps, th, tl);
+                    a.resume[fid] = pack_resume(th, tl, pf, steps, sign0, false, phase);
+                    queue_push(a.queue + a.n, a.work + kWorkTailLen, fid);
+                    phase = PH_IDLE;
+                }
+                continue;
             }
         }
         const bool live = phase != PH_IDLE;
@@ -4122,10 +4148,10 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
             float nh, nl;
             t_after(t0, step, to, nh, nl);
             uint32_t decided = to;
+            ahead = 0;
             if (to < max_steps && t_less(nh, nl, far_t)) {
                 uint32_t g = (uint32_t)next;
                 if (g > 0u && mark_lo - to <= g + 1u) g = mark_lo - to > 2u ? mark_lo - to - 2u : 0u;
-                ahead = 0;
                 if (g > 0u) {
                     float ah, al;
                     t_after(t0, step, to + g, ah, al);
@@ -4427,10 +4453,10 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
     }
 }
 
-template <class Eval, bool RESUME, bool CERT = false>
+template <class Eval, bool RESUME, bool CERT = false, bool TAIL = false>
 __global__ void __launch_bounds__(256, Eval::kMinBlocks) k_march(FlightArgs a)
 {
-    march_flights<Eval, RESUME, CERT>(a);
+    march_flights<Eval, RESUME, CERT, TAIL>(a);
 }
 
 // The fast pass with two group sizes of one evaluator: batches of fewer than `few`
@@ -4967,6 +4993,7 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
     // from k_prepare; plain: every medium stationary with one octave
     b.setup_len = setup_len(a.one_d, a.max_imp, a.max_oct, a.any_ns, a.any_mr);
     const bool group1 = b.setup_len != 0u, plain = b.setup_len == 4u;
+    b.hand_over = 0u;
     b.run_lo = 0;
     b.run_hi = 0xffffffffu;
     if (!group1) b.setup = nullptr;     // the march kernels read set-up records only when written
@@ -5043,6 +5070,7 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
                 }, a.n_dev != nullptr);
             }
         }, [&] {
+            b.hand_over = plain ? (a.all_grid ? 0u : kHandOverPlain) : kHandOverGeneral;
             if (!plain) {
                 const void *fn = (const void *)k_march<EvalCoopOct, false>;
                 const size_t smem = smem_window(std::max<uint32_t>(a.max_oct, a.any_mr ? 2u : 1u));
@@ -5062,6 +5090,24 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
             }
         });
         if (failed != cudaSuccess) return failed;
+        if (b.hand_over != 0u) {
+            // the single-lane pass's last flights
+            if (plain) {
+                const void *fn = (const void *)k_march<EvalGroup1D<true, true>, false, false, true>;
+                k_march<EvalGroup1D<true, true>, false, false, true><<<grid(fn, 0, true, 8), 256, 0, stream>>>(b);
+            } else {
+                by_octaves(kFewWarps, [&] {
+                    const void *fn = (const void *)k_march<EvalWarp1D<true>, false, false, true>;
+                    k_march<EvalWarp1D<true>, false, false, true><<<grid(fn, 0, true, 32), 256, 0, stream>>>(b);
+                }, [&] {
+                    const void *fn = (const void *)k_march<EvalGroup1D<false, true>, false, false, true>;
+                    k_march<EvalGroup1D<false, true>, false, false, true><<<grid(fn, 0, true, 8), 256, 0, stream>>>(b);
+                }, true);
+                b.run_lo = 0;
+                b.run_hi = all;
+            }
+            b.hand_over = 0u;
+        }
     } else if (group3) {
         const void *fn = (const void *)k_march_sized<EvalGroup3D<32>, EvalGroup3D<8>>;
         cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemG3<8>);

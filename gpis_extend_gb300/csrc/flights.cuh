@@ -47,7 +47,8 @@ struct FlightArgs {
     uint4 *resume;              // scratch, n saved march states
     uint32_t *queue;            // scratch, 2 n flight indices (may be null: the resume passes then
                                 // scan every flight): the flights the fast pass hands on, then
-                                // those the certified resume pass hands on
+                                // those the certified resume pass hands on (before it runs, those
+                                // that wait for the fast pass's tail)
     int queue_in;               // set by launch_flights for each resume pass
     uint32_t setup_len;         // set by launch_flights: float4 per set-up record
     float4 *setup;              // scratch, setup_len() per flight: the march passes' per-flight set-up,
@@ -67,6 +68,8 @@ struct FlightArgs {
     uint32_t prop_cap;          // most steps one evaluation skips before a proposed interval (0: 32)
     uint32_t fast_window;       // stationary 1D fast pass: 0 impulse window in shared memory, 1 in registers
     uint32_t precise_only;      // 1: no certified resume pass (every crossing on the precise evaluator)
+    uint32_t hand_over;         // set by launch_flights: a single-lane fast pass whose flights have all been
+                                // pulled hands a warp's last so many on to the tail pass (0: none)
     uint32_t run_lo, run_hi;    // set by launch_flights: a march pass runs when its flight count, read on
                                 // the device, lies in [run_lo, run_hi)
     const uint32_t *n_dev;      // may be null: the live flight count in device memory (<= n,
