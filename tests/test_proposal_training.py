@@ -32,3 +32,20 @@ def test_gpu_gradient_at_tile_edges(n):
     for name, _ in R.PARAMS:
         rel = np.linalg.norm(gd[name] - gref[name]) / max(np.linalg.norm(gref[name]), 1e-12)
         assert rel <= 3e-2, (name, rel)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [1, 127, 128, 129, 1000])
+def test_gpu_features_at_block_edges(n):
+    """The features kernel stores a block's 128 rows together: every row up to n (bar of
+    test_gpu_features_match_restatement), nothing after the last."""
+    torch = pytest.importorskip("torch")
+    from gpis_extend_gb300 import runtime, workloads
+    desc = proposal.config2_medium()
+    b = workloads.torus_flights(n, desc)
+    with runtime.Context(desc) as ctx:
+        out = torch.full((n + 3, 24), 7.0, dtype=torch.float32, device="cuda")
+        f = runtime.proposal_features(ctx, runtime.DeviceFlights(b), out=out).cpu().numpy()
+    ref = R.features(desc, b.origin_near, b.dir_far, b.seeds, b.prev)
+    assert np.all(np.abs(f[:n] - ref) <= 1e-4 * (1 + np.abs(ref)))
+    assert np.all(f[n:] == 7.0)
