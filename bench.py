@@ -436,7 +436,10 @@ def learned_workload(args):
         "e2e": {"value": None, "unit": UNIT, "h2d_bytes_per_step": 0, "d2h_bytes_per_step": 0,
                 "note": "device-resident arms only; the host entry is measured by the default workload"},
         "learned": learned,
-        "gpu_launches": args.steps * 2 * 6,
+        # per batch: k_features, the inference, k_prepare, the fast pass, its tail and the
+        # precise pass (each launched in the forms for few and for many flights: 2 + 3; the
+        # form whose range the device count misses returns at once) and k_finish
+        "gpu_launches": args.steps * 2 * 10,
         "clocks": clocks.summary(),
     }
     prop.close()
@@ -767,9 +770,11 @@ def main():
                    "primary": prim.n, "secondary": sec.n, "l2": "inputs 512 MiB > L2 (no flush)",
                    "parallelism": f"replicas x{world} (disjoint flight ranges)", "schedule": schedule},
         "e2e": {"value": e2e_value, "unit": UNIT, "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
-        # per batch: k_prepare (the fast pass's set-up and the conditioning), the fast
-        # pass, the resume pass and k_finish; two batches per step
-        "gpu_launches": args.steps * 2 * 4,
+        # per batch: k_prepare (the passes' set-up and the conditioning), the fast pass, its
+        # tail, the certified and the precise pass (each launched in the forms for few and for
+        # many flights; the one whose range the queue misses returns at once) and k_finish;
+        # two batches per step
+        "gpu_launches": args.steps * 2 * 8,
         "roofline": roof,
         "counters": cnt,
         "clocks": clocks.summary(),

@@ -1,16 +1,20 @@
 // flights.cu -- sm_103a kernels of the GPIS ray-flight path.
 //
-// One batch of flights runs as three kernels on one stream:
+// One batch of flights runs on one stream:
 //   k_prepare  Renewal / Renewal+ conditioning at the origin of every
 //              secondary flight (SparseConvolutionNoise.cpp:488-656), one thread
-//              per flight, coefficients to a scratch record;
+//              per flight, coefficients to a scratch record; and, for 1D media of
+//              up to eight impulses, the march's per-flight set-up record;
 //   k_march    the first-sign-change march and regula-falsi back-off
 //              (SparseConvolutionNoiseMedium.cpp:287-346): persistent warps pull
 //              flights from a device work counter and refill finished lanes, so
 //              flights of very uneven length keep every lane busy; value-only
 //              field evaluations; the impulses of the cells around the query are kept
-//              and a cell is generated only when the query comes near it; 3D media give
-//              a flight to a group of lanes that share its impulses;
+//              and a cell is generated only when the query comes near it.  A fast pass
+//              with certified skips, for long 1D batches followed by its tail, then
+//              the certified pass (plain 1D media) and the precise pass over the
+//              flights handed on.  3D media, short 1D batches, tails and short queues
+//              give a flight to a group of lanes that share its impulses;
 //   k_finish   the gradient sample at the end point (evaluateGradient,
 //              SparseConvolutionNoise.cpp:133-296), one thread per flight.
 //
@@ -2176,12 +2180,12 @@ struct EvalGeneric {
     }
 };
 
-// The resume passes of batches whose media all use 1D noise: the generic evaluator
-// compiled for 4 blocks of 256 per SM (64 registers, with spills).  For the precise
-// pass that decides every crossing it hides the precise evaluator's dependent
-// float-float chains better than 2 blocks at 128 registers (15.93 against 16.57 ms
-// per bench step; 3 blocks: 16.07); the certified pass runs it too.  3D media keep
-// 2 blocks: their 27-cell evaluations spill too much at 64 registers.
+// The resume pass of 1D media with more than eight impulses per cell (the others resume
+// on lane groups): the generic evaluator compiled for 4 blocks of 256 per SM (64
+// registers, with spills).  Deciding every crossing it hides the precise evaluator's
+// dependent float-float chains better than 2 blocks at 128 registers (sphere field,
+// 15.93 against 16.57 ms per bench step; 3 blocks: 16.07).  3D media keep 2 blocks:
+// their 27-cell evaluations spill too much at 64 registers.
 struct EvalGeneric4 : EvalGeneric {
     static constexpr int kMinBlocks = 4;
 };
@@ -2849,9 +2853,9 @@ constexpr uint32_t kFewPlain = 32000, kFewGeneral = 20000;
 constexpr uint32_t kHandOverPlain = 8, kHandOverGeneral = 4;
 
 // STAT: every medium of the batch is stationary with one octave.  FAST: the fast pass,
-// whose sums keep the cooperative evaluators' order and which takes the slope along; the resume passes' values
-// keep the one-lane evaluators' order, so that a miss has the same bits whichever of them
-// ends it.
+// whose sums keep the cooperative evaluators' order and which takes the slope along; the
+// resume passes' values keep the one-lane evaluators' order, so that a miss has the same
+// bits whichever of them ends it.
 template <bool STAT, bool FAST>
 struct EvalGroup1D {
     static constexpr bool kCollective = false;
@@ -4997,13 +5001,11 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
     b.run_lo = 0;
     b.run_hi = 0xffffffffu;
     if (!group1) b.setup = nullptr;     // the march kernels read set-up records only when written
-    // hand-off queues only with the certified pass: a precise pass that takes a queue
-    // loads its flights in the order they were saved, scattered, and measured slower
-    // than one that scans every resume record in flight order (the uneven image batch
-    // 512 against 496 ms)
     const bool certify = plain && !a.all_grid && !a.precise_only;
     // stationary 3D media of up to 8 impulses per cell: lane groups, each of which loads
-    // its flight's record once for all its lanes, so the scattered order costs nothing
+    // its flight's record once for all its lanes, so a queue's scattered order costs
+    // nothing.  The one-lane evaluators of the other media scan every resume record in
+    // flight order instead (an uneven image batch 496 against 512 ms with a queue)
     const bool group3 = a.three_d && a.max_oct == 1 && !a.any_ns && !a.any_gen3d && a.max_imp <= (uint32_t)kG3Imp;
     if (!group1 && !group3) b.queue = nullptr;
     if (b.any_cond || b.setup) {

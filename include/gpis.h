@@ -295,9 +295,10 @@ int gpis_nee_host(gpis_ctx *ctx, const gpis_nee_soa *in, float *out, uint32_t n)
                                             one evaluation may skip before a flight's
                                             proposed interval, 8..256 (default 32; every
                                             skipped step is still certified)            */
-#define GPIS_TUNE_FAST_WINDOW       5u   /* stationary 1D fast pass: 0 (default) keeps
-                                            each lane's three-cell impulse window in
-                                            shared memory, 1 in registers              */
+#define GPIS_TUNE_FAST_WINDOW       5u   /* stationary 1D fast pass of long batches, one
+                                            lane per flight: 0 (default) keeps each
+                                            lane's three-cell impulse window in shared
+                                            memory, 1 in registers                     */
 #define GPIS_TUNE_PRECISE_DECISIONS 6u   /* 1: every crossing of a stationary 1D single-
                                             octave medium is decided on the precise
                                             evaluator; 0 (default): on fast values where
@@ -367,7 +368,7 @@ int gpis_se_splat_1d(const float *queries, const float *centers, float *values,
  * cudaFree can), or a plugin host that owns all device memory and forbids
  * plugins to allocate.  The same flight kernels as gpis_flights_submit run on
  * one medium description (no grid mean), with all working memory in a fixed
- * array of this library (about 12 MB for GPIS_STATIC_MAX_FLIGHTS flights)
+ * array of this library (about 16 MB for GPIS_STATIC_MAX_FLIGHTS flights)
  * that every GPU which loads the library keeps until the process exits.  The
  * caller provides device flight and result streams as for gpis_flights_submit.
  * Larger batches fail with GPIS_ERANGE.  The first call on a device, with that
@@ -457,7 +458,8 @@ typedef struct {
     uint64_t medium_events;
     uint64_t failed;            /* paths ended by a failed medium or phase sample */
     double ms;                  /* device time of the render (CUDA events)        */
-    uint64_t launches;          /* kernels launched by the render                 */
+    uint64_t launches;          /* kernels launched by the render (the passes of a
+                                   flight batch counted as one march and one resume) */
     uint64_t nee_queries;       /* neePDF / neeGrad queries of specular events    */
     uint32_t graphed;           /* 1: the bounce loop ran as a captured CUDA graph */
     uint32_t passes;            /* passes of up to 2^22 paths                     */
