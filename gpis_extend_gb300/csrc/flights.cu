@@ -2443,6 +2443,7 @@ struct EvalGroup3D {
     static constexpr bool kSkip = false;
     static_assert(G == 8 || G == 32, "eight lanes per cell: one cell at a time, or a row of three");
     float want, dlen, f_lo, f_hi;           // as EvalSkip3D
+    bool ranged;                            // some flight of this warp plans a range (warp-uniform)
     int cx, cy, cz;                         // the cell the block is centred on
     int rx, ry, rz;                         // its coordinates modulo 3
     bool valid;
@@ -2450,7 +2451,14 @@ struct EvalGroup3D {
     const PcgJump *sj;
     unsigned mask;
 
-    __device__ __forceinline__ void reset() { want = 0.0f; dlen = 0.0f; valid = false; cx = cy = cz = rx = ry = rz = 0; }
+    __device__ __forceinline__ void reset()
+    {
+        want = 0.0f;
+        dlen = 0.0f;
+        ranged = false;
+        valid = false;
+        cx = cy = cz = rx = ry = rz = 0;
+    }
     __device__ __forceinline__ void bind(const PcgJump *t)
     {
         extern __shared__ float4 dsm_g3[];
@@ -2633,7 +2641,7 @@ struct EvalGroup3D {
         Query q;
         locate(L, p, q);
         // the segment's end inside p's cell (EvalSkip3D)
-        if (len > 0.0f && m.skip_mean_lip >= 0.0f) {
+        if (len > 0.0f) {
 #pragma unroll
             for (int i = 0; i < 3; ++i) {
                 const float fr = q.t[i][1];
@@ -2643,16 +2651,14 @@ struct EvalGroup3D {
                 else if (di < 0.0f) room = (fr - kSupportEps) / -di;
                 len = fminf(len, room);
             }
-        } else {
-            len = 0.0f;
         }
         float v, lo = 0.0f, hi = 0.0f;
         const float E[3] = {len * d[0] / kr, len * d[1] / kr, len * d[2] / kr};
         const float ee = E[0] * E[0] + E[1] * E[1] + E[2] * E[2];
         const bool bound = len > 0.0f && ee > 0.0f;
-        // one of the groups of this warp wants a range: all of them run that form, which
+        // one of the groups of this warp plans a range: all of them run that form, which
         // costs less than both forms one after the other
-        if (__any_sync(__activemask(), bound)) {
+        if (ranged) {
             const float kr2 = kr * kr;
             const float kmax2 = fmaxf(fmaxf(m.kexp3d[0], m.kexp3d[1]), m.kexp3d[2]) * kr2;
             const float kmin2 = fminf(fminf(m.kexp3d[0], m.kexp3d[1]), m.kexp3d[2]) * kr2;
@@ -4062,6 +4068,16 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
             if (__all_sync(FULL, drained)) break;
             continue;
         }
+        if constexpr (kOwn3D) {
+            // a marching step of a 3D medium asks for the field's range over the next
+            // steps: about half of |f| at the last step, and at least two steps.  Whether
+            // some group of the warp does is voted on here, where all lanes meet: the two
+            // forms of the sums shuffle a different number of times, and the groups, and a
+            // group's own lanes, need not be converged later on
+            const float len = fminf(0.5f * fabsf(pf), (float)kMaxSkip3D * step);
+            ev.plan(live && phase == PH_MARCH && L.m->skip_mean_lip >= 0.0f && len >= 2.0f * step ? len : 0.0f);
+            ev.ranged = __any_sync(FULL, ev.want > 0.0f);
+        }
         if (!Eval::kCollective && !live) continue;
 
         // evaluation point of this phase
@@ -4079,10 +4095,8 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
         const bool precise = (!CERT && decide) ||
                              (std::is_same<Eval, EvalGeneric>::value && phase == PH_FAR && general_3d(*L.m));
         float margin = 0.0f;
-        if constexpr (IsSkip3D<Eval>::value) {
-            // a marching step of a 3D medium asks for the field's range over the next
-            // steps: about half of |f| at the last step, and at least two steps
-            if ((!RESUME || kOwn3D) && phase == PH_MARCH) {
+        if constexpr (IsSkip3D<Eval>::value && !kOwn3D) {
+            if (!RESUME && phase == PH_MARCH) {
                 const float len = fminf(0.5f * fabsf(pf), (float)kMaxSkip3D * step);
                 ev.plan(len >= 2.0f * step ? len : 0.0f);
             }
