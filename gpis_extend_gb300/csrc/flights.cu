@@ -132,7 +132,6 @@ struct MrLevels {
     uint32_t seed[2];
 };
 
-// FAST: the weights in float (within about 1e-7; the levels are the same).
 __device__ __noinline__ void level_weights_double(float frac, float &w0, float &w1)
 {
     const double f = (double)frac;
@@ -141,24 +140,23 @@ __device__ __noinline__ void level_weights_double(float frac, float &w0, float &
     w1 = (float)__ddiv_rn(f, den);
 }
 
-template <bool FAST = false>
-__device__ __forceinline__ MrLevels mr_levels(const DevMedium &m, float ls)
+// the levels around ls without their weights; ls's place between the two
+__device__ __forceinline__ float mr_scales(const DevMedium &m, float ls, MrLevels &r)
 {
     const float lv = floorf(__fdiv_rn(logf(ls), m.mr_log_base));
     int li = (int)lv;
     li = li < -kMrLevels ? -kMrLevels : (li > kMrLevels - 2 ? kMrLevels - 2 : li);
-    MrLevels r;
     r.s[0] = m.mr_pow[li + kMrLevels];
     r.s[1] = m.mr_pow[li + kMrLevels + 1];
     r.seed[0] = (uint32_t)m.mr_seed[li + kMrLevels];
     r.seed[1] = (uint32_t)m.mr_seed[li + kMrLevels + 1];
-    const float frac = __fdiv_rn(__fsub_rn(ls, r.s[0]), __fsub_rn(r.s[1], r.s[0]));
-    if (FAST) {
-        const float inv = rsqrtf(1.0f - 2.0f * frac + 2.0f * frac * frac);
-        r.w[0] = (1.0f - frac) * inv;
-        r.w[1] = frac * inv;
-        return r;
-    }
+    return __fdiv_rn(__fsub_rn(ls, r.s[0]), __fsub_rn(r.s[1], r.s[0]));
+}
+
+__device__ __forceinline__ MrLevels mr_levels(const DevMedium &m, float ls)
+{
+    MrLevels r;
+    const float frac = mr_scales(m, ls, r);
     if (!ffm_level_weights(frac, r.w[0], r.w[1])) level_weights_double(frac, r.w[0], r.w[1]);
     return r;
 }
@@ -2126,7 +2124,7 @@ __device__ __forceinline__ float value_1d(const LaneField &L, float px, float py
     const DevMedium &m = *L.m;
     float noise = 0.0f;
     if (m.flags & MF_MULTIRES) {
-        const MrLevels lv = mr_levels<true>(m, ls_value(m, px, pz));
+        const MrLevels lv = mr_levels(m, ls_value(m, px, pz));
 #pragma unroll 1
         for (int j = 0; j < 2; ++j) noise = __fmaf_rn(j ? lv.w[1] : lv.w[0], value_level(L, px, py, pz, j, lv, noise_at), noise);
         return __fmaf_rn(L.sigma, noise, lane_mean(L, px, py, pz, id));
@@ -2778,7 +2776,7 @@ __device__ __forceinline__ FastPoint fast_point(const LaneField &L, float px, fl
     q.bz = __fmul_rn(m.l_inv[2], pz);
     if (q.mr) {
         q.ls = ls_value(m, px, pz);
-        q.lv = mr_levels<true>(m, q.ls);
+        q.lv = mr_levels(m, q.ls);
         if (L.cond && lo.s != q.lv.s[0]) {
             lo.s = q.lv.s[0];
 #pragma unroll
@@ -3213,7 +3211,7 @@ struct EvalWarp1D {
             };
             float noise = 0.0f;
             if (m.flags & MF_MULTIRES) {
-                const MrLevels lv = mr_levels<true>(m, ls_value(m, px, pz));
+                const MrLevels lv = mr_levels(m, ls_value(m, px, pz));
                 const float nk = value_level(L, px, py, pz, i, lv, raw);
                 for (int k = 0; k < 2; ++k) noise = __fmaf_rn(k ? lv.w[1] : lv.w[0], __shfl_sync(FULL, nk, 8 * k), noise);
                 return __fmaf_rn(L.sigma, noise, lane_mean(L, px, py, pz, id));
@@ -3693,7 +3691,8 @@ __device__ __forceinline__ int oct_skip_count(const DevMedium &m, const LaneFiel
     const float dls = L.sk[1];
     const float reach = dls * ((float)cap * step) + 1e-6f;
     if (m.flags & MF_MULTIRES) {
-        const MrLevels lv = mr_levels<true>(m, ls_p);
+        MrLevels lv;
+        mr_scales(m, ls_p, lv);
         if (!(ls_p - reach > lv.s[0] * 1.00001f && ls_p + reach < lv.s[1] * 0.99999f)) return 0;
         const float is = __fdividef(1.0f, lv.s[0]);
         lip += 1.0771f * m.skip_noise_lip * is * L.sk[3] + 1.4143f * (0.42888194f * is * L.sk[4] + 0.5f * L.sk[5]) +
