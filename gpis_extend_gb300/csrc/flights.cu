@@ -2786,7 +2786,7 @@ __device__ __forceinline__ FastPoint fast_point(const LaneField &L, float px, fl
         q.oz[1] = lo.oz[1];
     } else if (m.ls_kind) {
         q.ls = ns_scale(m, px, pz);
-        q.kexp = __fdividef(q.kexp, q.ls * q.ls);
+        q.kexp = __fdiv_rn(q.kexp, q.ls * q.ls);
         q.inv_norm = inv_norm_1d(m, q.ls);
         q.ca = splat_cov_1d(q.ls, L.ls_o);
         q.bx = __fdiv_rn(q.bx, m.ls_max);
