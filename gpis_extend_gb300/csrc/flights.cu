@@ -3791,11 +3791,11 @@ __device__ __forceinline__ float skip_scale(const DevMedium &m, float px, float 
     return (m.flags & MF_MULTIRES) ? ls_value(m, px, pz) : ns_scale(m, px, pz);
 }
 
-// the evaluators whose fast pass skips by oct_skip_count, and the cap of each
-template <class E> struct IsOct { static constexpr bool value = false; static constexpr int cap = 0; };
-template <> struct IsOct<EvalCoopOct> { static constexpr bool value = true; static constexpr int cap = 16; };
-template <> struct IsOct<EvalWarp1D<true>> { static constexpr bool value = true; static constexpr int cap = 16; };
-template <> struct IsOct<EvalGroup1D<false, true>> { static constexpr bool value = true; static constexpr int cap = 16; };
+// the evaluators whose fast pass skips by oct_skip_count
+template <class E> struct IsOct { static constexpr bool value = false; };
+template <> struct IsOct<EvalCoopOct> { static constexpr bool value = true; };
+template <> struct IsOct<EvalWarp1D<true>> { static constexpr bool value = true; };
+template <> struct IsOct<EvalGroup1D<false, true>> { static constexpr bool value = true; };
 
 template <class E> struct IsSkip3D { static constexpr bool value = false; };
 template <> struct IsSkip3D<EvalSkip3D> { static constexpr bool value = true; };
@@ -3818,10 +3818,6 @@ __device__ __forceinline__ float eval_at(EvalGroup3D<G> &ev, const LaneField &L,
 {
     return ev.value(L, d, p[0], p[1], p[2], id, refills, live);
 }
-// before a proposed crossing interval the cap is this by default (every skipped step is
-// still certified; GPIS_TUNE_PROPOSED_SKIP_CAP sets it)
-constexpr int kMaxSkipProposed = 32;
-
 // Fast values farther than this from zero have the sign of the precise value
 // (the fast evaluator differs from the precise one by a few 1e-8).
 constexpr float kPreciseBand = 1e-6f;
@@ -3968,7 +3964,9 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
     float prop_a = -INFINITY;   // start of the proposed crossing interval (learned proposal)
     // certified pass: the bound on fac's distance from the reference's (cert_fac)
     float dfac = 0.0f;
-    const int prop_cap = a.prop_cap ? (int)a.prop_cap : kMaxSkipProposed;
+    // before a proposed crossing interval the limit of the reach is GPIS_TUNE_PROPOSED_SKIP_CAP,
+    // where that is set (every skipped step is certified whatever it is)
+    const int prop_cap = a.prop_cap ? (int)a.prop_cap : kMaxReach;
     // the flights this pass takes: every flight, or the queue the pass before filled
     const int q_in = TAIL ? 2 : (RESUME && a.queue ? a.queue_in : 0);
     const uint32_t *queue_in = q_in ? a.queue + (size_t)(q_in - 1) * a.n : nullptr;
@@ -4157,17 +4155,15 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
         // the steps that the value f at step idx (0: nearT) decides, and the next one to evaluate
         auto advance = [&](uint32_t idx) {
             int back = 0, fore = 0, next = 0;   // steps decided before and after, and the next one's lead
-            const bool early = th < prop_a;
+            const int limit = th < prop_a ? prop_cap : kMaxReach;
             if constexpr (Eval::kSkip) {
-                reach_1d(L, d, p, f, sg, ev.slope * L.sigma * dzdt, curv, jump0, jump1, dzdt, step,
-                         early ? max(prop_cap, kMaxReach) : kMaxReach, back, fore);
+                reach_1d(L, d, p, f, sg, ev.slope * L.sigma * dzdt, curv, jump0, jump1, dzdt, step, limit, back, fore);
                 next = min(back, fore);
             }
             if constexpr (IsOct<Eval>::value) {
                 // the bound takes the worst local scale of the span, so the span follows
-                // the last reach
-                const int cap = min(max(2 * reach + 2, 4), kMaxReach);
-                back = fore = oct_skip_count(*L.m, L, ev.last_ls, f, step, early ? max(cap, prop_cap) : cap);
+                // the last reach, before a proposed interval too
+                back = fore = oct_skip_count(*L.m, L, ev.last_ls, f, step, min(max(2 * reach + 2, 4), limit));
                 reach = fore;
                 next = (3 * fore) >> 2;
             }
@@ -4353,17 +4349,19 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                 // steps are counted as marched; the resume pass re-evaluates the step before
                 // a crossing, so no skipped value is ever needed.
                 int skip = 0;
+                const bool early = th < prop_a;
                 if constexpr (Eval::kSkip) {
                     float lip, j0, j1;
                     skip_params(*L.m, d, L.sigma, L.cond, L.vs, L.gsz, step, lip, j0, j1);
                     const float af = fabsf(f) * (1.0f - 1e-6f) - 1e-5f - j0, per = lip * step + j1;
-                    if (lip >= 0.0f && af > per) skip = (int)fminf(af / per, (float)kMaxSkip);
+                    if (lip >= 0.0f && af > per) skip = (int)fminf(af / per, (float)(early ? prop_cap : kMaxSkip));
                 }
                 if constexpr (IsSkip3D<Eval>::value) {
                     if (!RESUME || kOwn3D) skip = ev.skips(f, step, kMaxSkip3D);
                 }
                 if constexpr (IsOct<Eval>::value) {
-                    if (!RESUME) skip = oct_skip_count(*L.m, L, ev.last_ls, f, step, IsOct<Eval>::cap);
+                    // (a longer span loosens the bound, whatever a proposal says)
+                    if (!RESUME) skip = oct_skip_count(*L.m, L, ev.last_ls, f, step, early ? min(prop_cap, kMaxSkip) : kMaxSkip);
                 }
                 if constexpr (RESUME) {
                     // a flight that marches on after a decision skips by the same slope bound
