@@ -2449,6 +2449,7 @@ struct EvalGroup3D {
     float4 *cells;                          // the group's 27 x 8 impulses: position, weight
     const PcgJump *sj;
     unsigned mask;
+    uint32_t drawn;                         // cells drawn, counted by the group's first lane
 
     __device__ __forceinline__ void reset()
     {
@@ -2464,6 +2465,7 @@ struct EvalGroup3D {
         cells = dsm_g3 + (threadIdx.x / G) * (27 * kG3Imp);
         sj = t;
         mask = group_mask(G);
+        drawn = 0u;
     }
     __device__ __forceinline__ void plan(float len) { want = len; }
 
@@ -2527,6 +2529,7 @@ struct EvalGroup3D {
         cy = y;
         cz = z;
         valid = true;
+        if ((threadIdx.x & (G - 1)) == 0) drawn += near_by ? 9u : 27u;
         __syncwarp(mask);       // every lane has read the old block
         draw(near_by ? 9 : 27, m, seed, [&](int j, int &ox, int &oy, int &oz) {
             const int a = j / 9, b = (j / 3) % 3 - 1, c = j % 3 - 1;
@@ -2628,10 +2631,9 @@ struct EvalGroup3D {
     }
 
     __device__ __forceinline__ float value(const LaneField &L, const float d[3], float px, float py, float pz, int &id,
-                                           uint32_t &refills, bool)
+                                           uint32_t &, bool)
     {
         const DevMedium &m = *L.m;
-        refills += 27;
         const float p[3] = {px, py, pz};
         float len = want;
         want = 0.0f;
@@ -2899,6 +2901,8 @@ struct EvalGroup1D {
     const PcgJump *sj;
     float4 *terms;          // the group's 24 terms
     unsigned mask;
+    uint32_t drawn;         // cells drawn, counted by the group's first lane
+    bool spare;             // repeats another group's cells: not counted
 
     __device__ __forceinline__ void reset() { valid = 0u; last_ls = 1.0f; slope = 0.0f; lo = {}; }
     __device__ __forceinline__ void bind(const PcgJump *t)
@@ -2907,6 +2911,8 @@ struct EvalGroup1D {
         terms = s_terms + (threadIdx.x >> 3) * 6;
         sj = t;
         mask = group_mask(8);
+        drawn = 0u;
+        spare = false;
     }
 
     __device__ __forceinline__ float draw(int cell, uint32_t seed, uint32_t n_imp) const
@@ -2927,6 +2933,7 @@ struct EvalGroup1D {
             if (kWin > 1 && o != j) continue;
             const bool ok = ((valid >> o) & 1u) && wseed[o] == seed;
             if (!ok || ci != base[o]) {
+                if ((threadIdx.x & 7) == 0 && !spare) drawn += ok && (ci == base[o] + 1 || ci == base[o] - 1) ? 1u : 3u;
                 if (ok && ci == base[o] + 1) {
                     w[o][0] = w[o][1];
                     w[o][1] = w[o][2];
@@ -3046,11 +3053,9 @@ struct EvalGroup1D {
     {
         if constexpr (STAT && !FAST) {
             float margin;
-            refills += 3;
-            return certified(L, px, py, pz, id, margin);
+            return certified(L, px, py, pz, id, margin, refills);
         } else if constexpr (STAT) {
             const float z = ray_coord(L.li, L.n, px, py, pz);
-            refills += 3;
             float der;
             float noise = raw_sum<false>(*L.m, 0, z, L.seed, 1.0f, nullptr, &der) * L.inv_norm;
             slope = -L.kr * der * L.inv_norm;
@@ -3068,13 +3073,11 @@ struct EvalGroup1D {
 #pragma unroll 1
             for (int o = 0; o < n_oct; ++o) {
                 const float z = fast_coord(L, q, o);
-                refills += 3;
                 total = __fadd_rn(total, fast_share(L, q, o, z, octave_sum(L, o, z, fast_seed(L, q, o), q.kexp)));
             }
             return total + lane_mean(L, px, py, pz, id);
         } else {
             return value_1d(L, px, py, pz, id, [&](int j, float z, uint32_t seed, float ls) {
-                refills += 3;
                 return raw_sum<false>(*L.m, j, z, seed, ls, nullptr);
             });
         }
@@ -3090,7 +3093,7 @@ struct EvalGroup1D {
     }
 
     __device__ __forceinline__ float certified(const LaneField &L, float px, float py, float pz, int &id, float &margin,
-                                               bool = true)
+                                               uint32_t &, bool = true)
     {
         return value_1d_cert(L, px, py, pz, id, [&](float z, uint32_t seed, float ls) {
             return raw_sum<true>(*L.m, 0, z, seed, ls, &margin);
@@ -3183,18 +3186,19 @@ struct EvalWarp1D {
                 oz = L.c3.oct[k].gs[0];
             }
     }
-    __device__ __forceinline__ int octave(const DevMedium &m) const
+    // the eights beyond the last octave repeat it
+    __device__ __forceinline__ int octave(const DevMedium &m)
     {
-        return min(o, (m.flags & MF_MULTIRES) ? 1 : (int)m.n_oct - 1);
+        const int last = (m.flags & MF_MULTIRES) ? 1 : (int)m.n_oct - 1;
+        part.spare = o > last;
+        return min(o, last);
     }
 
-    __device__ __forceinline__ float value(const LaneField &L, float px, float py, float pz, int &id, uint32_t &refills,
-                                           bool)
+    __device__ __forceinline__ float value(const LaneField &L, float px, float py, float pz, int &id, uint32_t &, bool)
     {
         const DevMedium &m = *L.m;
         const int i = octave(m);
         float vs, gz, oz;
-        refills += 3;
         if constexpr (FAST) {
             const FastPoint q = fast_point(L, px, py, pz, lo);
             last_ls = q.ls;
@@ -3410,11 +3414,10 @@ struct EvalCoop1D {
     // the certified pass's value (value_1d_cert): noise1d_generic's order of the sum, and the
     // margin to the nearest support edge or cell face
     __device__ __forceinline__ float certified(const LaneField &L, float px, float py, float pz, int &id, float &margin,
-                                               bool live)
+                                               uint32_t &refills, bool live)
     {
         static_assert(SM, "the certified pass keeps its windows in shared memory");
         return value_1d_cert(L, px, py, pz, id, [&](float z, uint32_t, float) {
-            uint32_t refills = 0u;
             const float frac = locate(L, z, refills, live);
             float mg = fminf(frac, 1.0f - frac), sv = 0.0f;
             each_term(frac, L.kexp, [&](int, float tp, float w) {
@@ -3882,6 +3885,12 @@ __device__ __forceinline__ void t_after(float t0, float step, uint32_t k, float 
     lo = __fsub_rn(l, __fsub_rn(hi, s));
 }
 
+// the cells a lane group's evaluator drew, in the lane that counted them
+template <class Eval>
+__device__ __forceinline__ uint32_t cells_drawn(const Eval &ev) { return ev.drawn; }
+template <bool FAST>
+__device__ __forceinline__ uint32_t cells_drawn(const EvalWarp1D<FAST> &ev) { return ev.part.drawn; }
+
 __device__ __forceinline__ unsigned long long warp_sum(uint32_t v)
 {
     unsigned long long x = v;
@@ -4134,8 +4143,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
         if constexpr (CERT) {
             // every phase on the one evaluator (its value is EvalGeneric's), so that
             // the lanes of a warp never run two
-            f = ev.certified(L, p[0], p[1], p[2], id, margin, live);
-            c_refills += 3;
+            f = ev.certified(L, p[0], p[1], p[2], id, margin, c_refills, live);
         } else {
             if constexpr (G > 1) {
                 f = precise ? ev.precise(L, p, id) : eval_at(ev, L, d, p, id, c_refills, live);
@@ -4479,6 +4487,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
         }
     }
     // counters: one atomic per warp
+    if constexpr (G > 1) c_refills += cells_drawn(ev);
     const unsigned long long s0 = warp_sum(c_flights), s1 = warp_sum(c_steps), s2 = warp_sum(c_refine),
                              s3 = warp_sum(c_hits), s4 = warp_sum(c_limit), s5 = warp_sum(c_invalid),
                              s6 = warp_sum(c_refills), s7 = warp_sum(c_skipped);

@@ -163,7 +163,8 @@ typedef struct gpis_counters {
     uint64_t hits;
     uint64_t step_limit;
     uint64_t invalid;
-    uint64_t cell_refills;      /* impulse-cache cell regenerations                */
+    uint64_t cell_refills;      /* cells whose impulses were drawn: into a flight's window
+                                   or, by evaluators without one, at an evaluation */
     uint64_t skipped_steps;     /* march steps decided by the field bound, unevaluated */
 } gpis_counters;
 
