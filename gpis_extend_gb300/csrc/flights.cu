@@ -132,12 +132,16 @@ struct MrLevels {
     uint32_t seed[2];
 };
 
-__device__ __noinline__ void level_weights_double(float frac, float &w0, float &w1)
+// Float-float with a test of the rounding, the double evaluation for the values it cannot
+// decide; out of line, so that the march kernels of media without levels carry none of it
+// (three octaves, 300 007 flights: 9.05 ms a batch with it inline).
+__device__ __forceinline__ float2 level_weights(float frac)
 {
+    float w0, w1;
+    if (ffm_level_weights(frac, w0, w1)) return make_float2(w0, w1);
     const double f = (double)frac;
     const double den = __dsqrt_rn(__dadd_rn(__dsub_rn(1.0, __dmul_rn(2.0, f)), __dmul_rn(__dmul_rn(2.0, f), f)));
-    w0 = (float)__ddiv_rn(__dsub_rn(1.0, f), den);
-    w1 = (float)__ddiv_rn(f, den);
+    return make_float2((float)__ddiv_rn(__dsub_rn(1.0, f), den), (float)__ddiv_rn(f, den));
 }
 
 // the levels around ls without their weights; ls's place between the two
@@ -156,8 +160,9 @@ __device__ __forceinline__ float mr_scales(const DevMedium &m, float ls, MrLevel
 __device__ __forceinline__ MrLevels mr_levels(const DevMedium &m, float ls)
 {
     MrLevels r;
-    const float frac = mr_scales(m, ls, r);
-    if (!ffm_level_weights(frac, r.w[0], r.w[1])) level_weights_double(frac, r.w[0], r.w[1]);
+    const float2 w = level_weights(mr_scales(m, ls, r));
+    r.w[0] = w.x;
+    r.w[1] = w.y;
     return r;
 }
 
@@ -2449,7 +2454,6 @@ struct EvalGroup3D {
     float4 *cells;                          // the group's 27 x 8 impulses: position, weight
     const PcgJump *sj;
     unsigned mask;
-    uint32_t drawn;                         // cells drawn, counted by the group's first lane
 
     __device__ __forceinline__ void reset()
     {
@@ -2465,7 +2469,6 @@ struct EvalGroup3D {
         cells = dsm_g3 + (threadIdx.x / G) * (27 * kG3Imp);
         sj = t;
         mask = group_mask(G);
-        drawn = 0u;
     }
     __device__ __forceinline__ void plan(float len) { want = len; }
 
@@ -2511,7 +2514,7 @@ struct EvalGroup3D {
     }
 
     // the block of 27 cells around (x, y, z)
-    __device__ __forceinline__ void move(int x, int y, int z, const DevMedium &m, uint32_t seed)
+    __device__ __forceinline__ void move(int x, int y, int z, const DevMedium &m, uint32_t seed, uint32_t &refills)
     {
         if (valid && x == cx && y == cy && z == cz) return;
         // one step along one axis (within the range where x + 1 does not wrap): the
@@ -2529,7 +2532,7 @@ struct EvalGroup3D {
         cy = y;
         cz = z;
         valid = true;
-        if ((threadIdx.x & (G - 1)) == 0) drawn += near_by ? 9u : 27u;
+        refills += near_by ? 9u : 27u;
         __syncwarp(mask);       // every lane has read the old block
         draw(near_by ? 9 : 27, m, seed, [&](int j, int &ox, int &oy, int &oz) {
             const int a = j / 9, b = (j / 3) % 3 - 1, c = j % 3 - 1;
@@ -2544,7 +2547,7 @@ struct EvalGroup3D {
         float t[3][3];          // fraction minus the cell offset, per axis
         int sx[3], sy[3], sz[3];  // slot of each offset
     };
-    __device__ __forceinline__ void locate(const LaneField &L, const float p[3], Query &q)
+    __device__ __forceinline__ void locate(const LaneField &L, const float p[3], Query &q, uint32_t &refills)
     {
         const DevMedium &m = *L.m;
         int c[3];
@@ -2557,7 +2560,7 @@ struct EvalGroup3D {
 #pragma unroll
             for (int o = 0; o < 3; ++o) q.t[i][o] = __fsub_rn(fr, (float)(o - 1));
         }
-        move(c[0], c[1], c[2], m, L.seed);
+        move(c[0], c[1], c[2], m, L.seed, refills);
 #pragma unroll
         for (int o = 0; o < 3; ++o) {
             q.sx[o] = wrap3(rx, o - 1) * 9;
@@ -2631,7 +2634,7 @@ struct EvalGroup3D {
     }
 
     __device__ __forceinline__ float value(const LaneField &L, const float d[3], float px, float py, float pz, int &id,
-                                           uint32_t &, bool)
+                                           uint32_t &refills, bool)
     {
         const DevMedium &m = *L.m;
         const float p[3] = {px, py, pz};
@@ -2640,7 +2643,7 @@ struct EvalGroup3D {
         dlen = 0.0f;
         const float kr = m.kr_world;
         Query q;
-        locate(L, p, q);
+        locate(L, p, q, refills);
         // the segment's end inside p's cell (EvalSkip3D)
         if (len > 0.0f) {
 #pragma unroll
@@ -2688,13 +2691,13 @@ struct EvalGroup3D {
         return range_skips(dlen, f_lo, f_hi, f, step, cap);
     }
 
-    __device__ __forceinline__ float precise(const LaneField &L, const float p[3], int &id)
+    __device__ __forceinline__ float precise(const LaneField &L, const float p[3], int &id, uint32_t &refills)
     {
         const DevMedium &m = *L.m;
         const float kr = m.kr_world;
         const int k = threadIdx.x & 7;
         Query q;
-        locate(L, p, q);
+        locate(L, p, q, refills);
         float sv = 0.0f;
         // a cell's impulse as noise3d_precise evaluates it; one that is out of reach adds
         // +0, which leaves a sum that started at +0 as it is
@@ -2746,17 +2749,22 @@ struct EvalGroup3D {
 struct FastPoint {
     bool mr;
     MrLevels lv;
-    float oz[2];                    // multi-resolution: the origin's coordinates at the two levels
+    float oz[2];
     float ls;                       // the local scale, as oct_skip_count takes it
     float kexp, inv_norm, ca;
     float bx, by, bz;               // the isotropic position (divided by the maximum lateral scale)
 };
+
+// (by selection: the octave may differ between the lanes)
+template <class T>
+__device__ __forceinline__ T pick2(const T (&v)[2], int o) { return o & 1 ? v[1] : v[0]; }
 
 // The origin's coordinates at a level's two scales, kept while the level stays (fast_point
 // takes six divisions for them; 60 013 flights 4.02 ms a batch where it did at every point).
 // They have the reference's bits: a coordinate of the same size is subtracted, 10^4 where a
 // scene lies a thousand units from the origin, and there the level-free coordinate divided
 // by the scale, an ulp or two off, decided 0.8 % of short conditioned flights wrongly.
+// In shared memory: in registers they made the kernels spill for media without levels too.
 struct LevelOrigin {
     float s;                        // the lower level's scale (0: none)
     float oz[2];
@@ -2779,10 +2787,12 @@ __device__ __forceinline__ FastPoint fast_point(const LaneField &L, float px, fl
     if (q.mr) {
         q.ls = ls_value(m, px, pz);
         q.lv = mr_levels(m, q.ls);
-        if (L.cond && lo.s != q.lv.s[0]) {
-            lo.s = q.lv.s[0];
+        if (L.cond) {
+            if (lo.s != q.lv.s[0]) {
+                lo.s = q.lv.s[0];
 #pragma unroll
-            for (int j = 0; j < 2; ++j) lo.oz[j] = ray_coord_oct(m, L.n, L.o[0], L.o[1], L.o[2], q.lv.s[j]);
+                for (int j = 0; j < 2; ++j) lo.oz[j] = ray_coord_oct(m, L.n, L.o[0], L.o[1], L.o[2], q.lv.s[j]);
+            }
         }
         q.oz[0] = lo.oz[0];
         q.oz[1] = lo.oz[1];
@@ -2797,10 +2807,6 @@ __device__ __forceinline__ FastPoint fast_point(const LaneField &L, float px, fl
     }
     return q;
 }
-
-// (by selection: the octave may differ between the lanes)
-template <class T>
-__device__ __forceinline__ T pick2(const T (&v)[2], int o) { return o & 1 ? v[1] : v[0]; }
 
 // each octave divides the position by its length multiplier, a multiply when that is a
 // power of two (the same rounding as ray_coord_oct's division)
@@ -2901,8 +2907,6 @@ struct EvalGroup1D {
     const PcgJump *sj;
     float4 *terms;          // the group's 24 terms
     unsigned mask;
-    uint32_t drawn;         // cells drawn, counted by the group's first lane
-    bool spare;             // repeats another group's cells: not counted
 
     __device__ __forceinline__ void reset() { valid = 0u; last_ls = 1.0f; slope = 0.0f; lo = {}; }
     __device__ __forceinline__ void bind(const PcgJump *t)
@@ -2911,8 +2915,6 @@ struct EvalGroup1D {
         terms = s_terms + (threadIdx.x >> 3) * 6;
         sj = t;
         mask = group_mask(8);
-        drawn = 0u;
-        spare = false;
     }
 
     __device__ __forceinline__ float draw(int cell, uint32_t seed, uint32_t n_imp) const
@@ -2925,26 +2927,28 @@ struct EvalGroup1D {
         return __uint_as_float(__float_as_uint(unit_float(r1)) | (~r2 & 0x80000000u));
     }
 
-    // the window of octave or level j around cell ci
-    __device__ __forceinline__ void window(int j, int ci, uint32_t seed, uint32_t n_imp, float c[3])
+    // the window of octave or level j around cell ci (every lane counts the cells drawn)
+    __device__ __forceinline__ void window(int j, int ci, uint32_t seed, uint32_t n_imp, float c[3], uint32_t &refills)
     {
 #pragma unroll
         for (int o = 0; o < kWin; ++o) {
             if (kWin > 1 && o != j) continue;
             const bool ok = ((valid >> o) & 1u) && wseed[o] == seed;
             if (!ok || ci != base[o]) {
-                if ((threadIdx.x & 7) == 0 && !spare) drawn += ok && (ci == base[o] + 1 || ci == base[o] - 1) ? 1u : 3u;
                 if (ok && ci == base[o] + 1) {
                     w[o][0] = w[o][1];
                     w[o][1] = w[o][2];
                     w[o][2] = draw(ci + 1, seed, n_imp);
+                    refills += 1u;
                 } else if (ok && ci == base[o] - 1) {
                     w[o][2] = w[o][1];
                     w[o][1] = w[o][0];
                     w[o][0] = draw(ci - 1, seed, n_imp);
+                    refills += 1u;
                 } else {
 #pragma unroll
                     for (int d = 0; d < 3; ++d) w[o][d] = draw(ci + d - 1, seed, n_imp);
+                    refills += 3u;
                 }
                 base[o] = ci;
                 wseed[o] = seed;
@@ -2979,19 +2983,20 @@ struct EvalGroup1D {
     }
 
     // raw_sum of window 0 at the local scale ls
-    __device__ __forceinline__ float raw_sum_scaled(const DevMedium &m, float z, uint32_t seed, float ls)
+    __device__ __forceinline__ float raw_sum_scaled(const DevMedium &m, float z, uint32_t seed, float ls, uint32_t &refills)
     {
         const float tg = __fdiv_rn(z, m.kr_iso);
         const float fl = floorf(tg);
-        scale_terms(0, (int)fl, __fsub_rn(tg, fl), seed, m.n_imp, __fmul_rn(m.kexp1d, 1.0f / (ls * ls)));
+        scale_terms(0, (int)fl, __fsub_rn(tg, fl), seed, m.n_imp, __fmul_rn(m.kexp1d, 1.0f / (ls * ls)), refills);
         return row_sum();
     }
 
     // the terms of window o around cell ci, shared
-    __device__ __forceinline__ void scale_terms(int o, int ci, float frac, uint32_t seed, uint32_t n_imp, float kexp)
+    __device__ __forceinline__ void scale_terms(int o, int ci, float frac, uint32_t seed, uint32_t n_imp, float kexp,
+                                                uint32_t &refills)
     {
         float c[3], e[3];
-        window(o, ci, seed, n_imp, c);
+        window(o, ci, seed, n_imp, c, refills);
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
             const float tp = __fsub_rn(__fsub_rn(frac, (float)(d - 1)), fabsf(c[d]));
@@ -3018,13 +3023,13 @@ struct EvalGroup1D {
     // sum of e tp (by shuffles)
     template <bool MARGIN>
     __device__ __forceinline__ float raw_sum(const DevMedium &m, int j, float z, uint32_t seed, float ls, float *margin,
-                                             float *der = nullptr)
+                                             uint32_t &refills, float *der = nullptr)
     {
         const float tg = __fdiv_rn(z, m.kr_iso);
         const float fl = floorf(tg);
         const float frac = __fsub_rn(tg, fl);
         float c[3];
-        window(j, (int)fl, seed, m.n_imp, c);
+        window(j, (int)fl, seed, m.n_imp, c, refills);
         const float il2 = STAT ? 1.0f : 1.0f / (ls * ls);
         const float kexp = __fmul_rn(m.kexp1d, il2);
         float mg = fminf(frac, 1.0f - frac), e[3], dsum = 0.0f;
@@ -3057,7 +3062,7 @@ struct EvalGroup1D {
         } else if constexpr (STAT) {
             const float z = ray_coord(L.li, L.n, px, py, pz);
             float der;
-            float noise = raw_sum<false>(*L.m, 0, z, L.seed, 1.0f, nullptr, &der) * L.inv_norm;
+            float noise = raw_sum<false>(*L.m, 0, z, L.seed, 1.0f, nullptr, refills, &der) * L.inv_norm;
             slope = -L.kr * der * L.inv_norm;
             if (L.cond) {
                 const Cov1D k = cov1d(z - L.ozc);
@@ -3073,42 +3078,42 @@ struct EvalGroup1D {
 #pragma unroll 1
             for (int o = 0; o < n_oct; ++o) {
                 const float z = fast_coord(L, q, o);
-                total = __fadd_rn(total, fast_share(L, q, o, z, octave_sum(L, o, z, fast_seed(L, q, o), q.kexp)));
+                total = __fadd_rn(total, fast_share(L, q, o, z, octave_sum(L, o, z, fast_seed(L, q, o), q.kexp, refills)));
             }
             return total + lane_mean(L, px, py, pz, id);
         } else {
             return value_1d(L, px, py, pz, id, [&](int j, float z, uint32_t seed, float ls) {
-                return raw_sum<false>(*L.m, j, z, seed, ls, nullptr);
+                return raw_sum<false>(*L.m, j, z, seed, ls, nullptr, refills);
             });
         }
     }
 
     // the raw sum of octave o as EvalCoopOct adds it
-    __device__ __forceinline__ float octave_sum(const LaneField &L, int o, float z, uint32_t seed, float kexp)
+    __device__ __forceinline__ float octave_sum(const LaneField &L, int o, float z, uint32_t seed, float kexp, uint32_t &refills)
     {
         const float tg = __fdiv_rn(z, L.kr);
         const float fl = floorf(tg);
-        scale_terms(o, (int)fl, __fsub_rn(tg, fl), seed, L.n_imp, kexp);
+        scale_terms(o, (int)fl, __fsub_rn(tg, fl), seed, L.n_imp, kexp, refills);
         return pair_sum();
     }
 
     __device__ __forceinline__ float certified(const LaneField &L, float px, float py, float pz, int &id, float &margin,
-                                               uint32_t &, bool = true)
+                                               uint32_t &refills, bool = true)
     {
         return value_1d_cert(L, px, py, pz, id, [&](float z, uint32_t seed, float ls) {
-            return raw_sum<true>(*L.m, 0, z, seed, ls, &margin);
+            return raw_sum<true>(*L.m, 0, z, seed, ls, &margin, refills);
         });
     }
 
     // noise1d_precise
-    __device__ __forceinline__ float noise_precise(const DevMedium &m, int j, float z, uint32_t seed, float ls)
+    __device__ __forceinline__ float noise_precise(const DevMedium &m, int j, float z, uint32_t seed, float ls, uint32_t &refills)
     {
         const float kr = m.kr_iso;
         const float tg = __fdiv_rn(z, kr);
         const float fl = floorf(tg);
         const float frac = __fsub_rn(tg, fl);
         float c[3];
-        window(j, (int)fl, seed, m.n_imp, c);
+        window(j, (int)fl, seed, m.n_imp, c, refills);
         const float den = __fmul_rn(2.0f, __fmul_rn(ls, ls));
         float e[3];
 #pragma unroll
@@ -3136,10 +3141,10 @@ struct EvalGroup1D {
         return __fdiv_rn(sv, __fsqrt_rn(var));
     }
 
-    __device__ __forceinline__ float precise(const LaneField &L, const float p[3], int &id)
+    __device__ __forceinline__ float precise(const LaneField &L, const float p[3], int &id, uint32_t &refills)
     {
         return field_precise_1d(L, p[0], p[1], p[2], id, [&](int j, float z, uint32_t seed, float ls) {
-            return noise_precise(*L.m, j, z, seed, ls);
+            return noise_precise(*L.m, j, z, seed, ls, refills);
         });
     }
 };
@@ -3186,55 +3191,59 @@ struct EvalWarp1D {
                 oz = L.c3.oct[k].gs[0];
             }
     }
-    // the eights beyond the last octave repeat it
-    __device__ __forceinline__ int octave(const DevMedium &m)
+    __device__ __forceinline__ int octave(const DevMedium &m) const
     {
-        const int last = (m.flags & MF_MULTIRES) ? 1 : (int)m.n_oct - 1;
-        part.spare = o > last;
-        return min(o, last);
+        return min(o, (m.flags & MF_MULTIRES) ? 1 : (int)m.n_oct - 1);
     }
 
-    __device__ __forceinline__ float value(const LaneField &L, float px, float py, float pz, int &id, uint32_t &, bool)
+    __device__ __forceinline__ float value(const LaneField &L, float px, float py, float pz, int &id, uint32_t &refills,
+                                           bool)
     {
         const DevMedium &m = *L.m;
         const int i = octave(m);
+        uint32_t drawn = 0u;            // (the eights beyond the last octave repeat its cells)
         float vs, gz, oz;
         if constexpr (FAST) {
             const FastPoint q = fast_point(L, px, py, pz, lo);
             last_ls = q.ls;
             own(L, q.mr ? 0 : i, vs, gz, oz);
             const float z = fast_coord(L, q, i);
-            const float share = fast_share(L, q, i, z, part.octave_sum(L, 0, z, fast_seed(L, q, i), q.kexp), vs, gz, oz);
+            const float share = fast_share(L, q, i, z, part.octave_sum(L, 0, z, fast_seed(L, q, i), q.kexp, drawn), vs, gz, oz);
             float total = 0.0f;
             const int n = q.mr ? 2 : (int)m.n_oct;
             for (int k = 0; k < n; ++k) total = __fadd_rn(total, __shfl_sync(FULL, share, 8 * k));
+            refills += o == i ? drawn : 0u;
             return total + lane_mean(L, px, py, pz, id);
         } else {
             auto raw = [&](int, float z, uint32_t seed, float ls) {
-                return part.raw_sum_scaled(m, z, seed, ls);
+                return part.raw_sum_scaled(m, z, seed, ls, drawn);
             };
             float noise = 0.0f;
             if (m.flags & MF_MULTIRES) {
                 const MrLevels lv = mr_levels(m, ls_value(m, px, pz));
                 const float nk = value_level(L, px, py, pz, i, lv, raw);
+                refills += o == i ? drawn : 0u;
                 for (int k = 0; k < 2; ++k) noise = __fmaf_rn(k ? lv.w[1] : lv.w[0], __shfl_sync(FULL, nk, 8 * k), noise);
                 return __fmaf_rn(L.sigma, noise, lane_mean(L, px, py, pz, id));
             }
             own(L, i, vs, gz, oz);
             const float nk = value_octave(L, px, py, pz, i, ns_scale(m, px, pz), vs, gz, oz, raw);
+            refills += o == i ? drawn : 0u;
             for (int k = 0; k < (int)m.n_oct; ++k) noise = __fmaf_rn(oct_sigma(m, k), __shfl_sync(FULL, nk, 8 * k), noise);
             return __fadd_rn(noise, lane_mean(L, px, py, pz, id));
         }
     }
 
-    __device__ __forceinline__ float precise(const LaneField &L, const float p[3], int &id)
+    __device__ __forceinline__ float precise(const LaneField &L, const float p[3], int &id, uint32_t &refills)
     {
         const DevMedium &m = *L.m;
         const int i = octave(m);
-        auto noise_at = [&](int, float z, uint32_t seed, float ls) { return part.noise_precise(m, 0, z, seed, ls); };
+        uint32_t drawn = 0u;
+        auto noise_at = [&](int, float z, uint32_t seed, float ls) { return part.noise_precise(m, 0, z, seed, ls, drawn); };
         if (m.flags & MF_MULTIRES) {
             const MrLevels lv = mr_levels(m, ls_value_precise(m, p[0], p[2]));
             const float n = precise_level(L, p[0], p[1], p[2], i, lv, noise_at);
+            refills += o == i ? drawn : 0u;
             const float nb = __fadd_rn(__fmul_rn(lv.w[0], __shfl_sync(FULL, n, 0)), __fmul_rn(lv.w[1], __shfl_sync(FULL, n, 8)));
             return mean_plus_precise(m, __fmul_rn(L.sigma, nb), p[0], p[1], p[2], id);
         }
@@ -3242,6 +3251,7 @@ struct EvalWarp1D {
         float vs, gz, oz;
         own(L, i, vs, gz, oz);
         const float n = precise_octave(L, p[0], p[1], p[2], i, ls, L.cond ? precise_den2(m, L, ls) : 0.0f, vs, gz, oz, noise_at);
+        refills += o == i ? drawn : 0u;
         float an = 0.0f;
         for (int k = 0; k < (int)m.n_oct; ++k) {
             const float nk = __shfl_sync(FULL, n, 8 * k);
@@ -3885,12 +3895,6 @@ __device__ __forceinline__ void t_after(float t0, float step, uint32_t k, float 
     lo = __fsub_rn(l, __fsub_rn(hi, s));
 }
 
-// the cells a lane group's evaluator drew, in the lane that counted them
-template <class Eval>
-__device__ __forceinline__ uint32_t cells_drawn(const Eval &ev) { return ev.drawn; }
-template <bool FAST>
-__device__ __forceinline__ uint32_t cells_drawn(const EvalWarp1D<FAST> &ev) { return ev.part.drawn; }
-
 __device__ __forceinline__ unsigned long long warp_sum(uint32_t v)
 {
     unsigned long long x = v;
@@ -4146,7 +4150,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
             f = ev.certified(L, p[0], p[1], p[2], id, margin, c_refills, live);
         } else {
             if constexpr (G > 1) {
-                f = precise ? ev.precise(L, p, id) : eval_at(ev, L, d, p, id, c_refills, live);
+                f = precise ? ev.precise(L, p, id, c_refills) : eval_at(ev, L, d, p, id, c_refills, live);
             } else
             f = precise ? field_precise(L, p[0], p[1], p[2], id)
                         : (use3 ? ev3.value(L, d, p[0], p[1], p[2], id, c_refills, live)
@@ -4486,8 +4490,9 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
             phase = PH_IDLE;
         }
     }
-    // counters: one atomic per warp
-    if constexpr (G > 1) c_refills += cells_drawn(ev);
+    // counters: one atomic per warp.  (A group's lanes have each counted the cells it drew;
+    // the eights of a warp per flight, which hold an octave each, their own.)
+    if (G > 1 && (lane & (kOwn3D ? G - 1 : 7)) != 0) c_refills = 0u;
     const unsigned long long s0 = warp_sum(c_flights), s1 = warp_sum(c_steps), s2 = warp_sum(c_refine),
                              s3 = warp_sum(c_hits), s4 = warp_sum(c_limit), s5 = warp_sum(c_invalid),
                              s6 = warp_sum(c_refills), s7 = warp_sum(c_skipped);
