@@ -174,21 +174,24 @@ __global__ void k_prep(const float *feat, uint32_t n, bf *xb, bf *ub, float *h0,
     }
 }
 
-// GRU cell (PyTorch gate order r, z, n) from the raw products gi = x W_ih^T, gh = h W_hh^T.
-__global__ void k_gru_cell(const float *gi, const float *gh, const float *P, const float *hprev, uint32_t n,
-                           float *r_o, float *z_o, float *n_o, float *ghn_o, float *hnew, bf *hnewb, bf *ub)
+// GRU cell (PyTorch gate order r, z, n) from the raw products gi = x W_ih^T, gh = h W_hh^T;
+// the gates r, z, n take gi's place (a thread's three values each).
+__global__ void k_gru_cell(float *gi, const float *gh, const float *P, const float *hprev, uint32_t n, float *ghn_o,
+                           float *hnew, bf *hnewb, bf *ub)
 {
     const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n * HID) return;
     const uint32_t m = i / HID, c = i % HID;
     const float *bih = P + O_BIH, *bhh = P + O_BHH;
-    const float *a = gi + (size_t)m * 3 * HID, *b = gh + (size_t)m * 3 * HID;
+    float *a = gi + (size_t)m * 3 * HID;
+    const float *b = gh + (size_t)m * 3 * HID;
     const float r = sigm(a[c] + bih[c] + b[c] + bhh[c]);
     const float z = sigm(a[HID + c] + bih[HID + c] + b[HID + c] + bhh[HID + c]);
     const float ghn = b[2 * HID + c] + bhh[2 * HID + c];
     const float nn = tanhf(a[2 * HID + c] + bih[2 * HID + c] + r * ghn);
     const float h = (1.0f - z) * nn + z * hprev[i];
-    r_o[i] = r; z_o[i] = z; n_o[i] = nn; ghn_o[i] = ghn;
+    a[c] = r; a[HID + c] = z; a[2 * HID + c] = nn;
+    ghn_o[i] = ghn;
     hnew[i] = h;
     hnewb[i] = __float2bfloat16_rn(h);
     if (ub) ub[(size_t)m * MLPIN + c] = __float2bfloat16_rn(h);
@@ -317,24 +320,30 @@ __global__ void __launch_bounds__(256) k_gelu_back(const float *dy, const float 
 }
 
 // one GRU step backward: gate gradients (BF16), dh * z, and the sums of the gate
-// gradients over the rows (b_ih: r, z, n; b_hh: r, z, n * r)
-__global__ void __launch_bounds__(256) k_gru_back(const float *dh, long ldh, const float *r_, const float *z_,
-                                                  const float *n_, const float *ghn_, const float *hprev, uint32_t n,
-                                                  bf *dgib, bf *dghb, float *dhpart, float *dbih, float *dbhh)
+// gradients over the rows (b_ih: r, z, n; b_hh: r, z, n * r).  The two rows of 96 BF16 gate
+// gradients (with respect to the input's and the state's products) take the place of their
+// row of 96 FP32 gates: a row is one warp's, which has read all of it before it writes.  Gates
+// and gradients of all eight steps side by side took 14.8 KB a flight, this 8.6.
+constexpr int kGateRow = 2 * 3 * HID;   // BF16 values of such a row
+__global__ void __launch_bounds__(256) k_gru_back(const float *dh, long ldh, float *gates, const float *ghn_,
+                                                  const float *hprev, uint32_t n, float *dhpart, float *dbih, float *dbhh)
 {
+    static_assert(HID == 32, "a row of gates is read and written by one warp");
     __shared__ float4 part[256];
     const int c = threadIdx.x % HID;
     float4 sum = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     for (size_t m = (size_t)blockIdx.x * (256 / HID) + threadIdx.x / HID; m < n; m += (size_t)gridDim.x * (256 / HID)) {
         const size_t i = m * HID + c;
         const float d = dh[m * ldh + c];
-        const float r = r_[i], z = z_[i], nn = n_[i], ghn = ghn_[i];
+        float *row = gates + m * 3 * HID;
+        const float r = row[c], z = row[HID + c], nn = row[2 * HID + c], ghn = ghn_[i];
+        __syncwarp();
         const float dz = d * (hprev[i] - nn) * z * (1.0f - z);
         const float dn = d * (1.0f - z) * (1.0f - nn * nn);
         const float dr = dn * ghn * r * (1.0f - r);
         const float dnr = dn * r;
         sum.x += dr; sum.y += dz; sum.z += dn; sum.w += dnr;
-        bf *gib = dgib + m * 3 * HID, *ghb = dghb + m * 3 * HID;
+        bf *gib = reinterpret_cast<bf *>(row), *ghb = gib + 3 * HID;
         const bf br = __float2bfloat16_rn(dr), bz = __float2bfloat16_rn(dz);
         gib[c] = br; gib[HID + c] = bz; gib[2 * HID + c] = __float2bfloat16_rn(dn);
         ghb[c] = br; ghb[HID + c] = bz; ghb[2 * HID + c] = __float2bfloat16_rn(dnr);
@@ -1166,8 +1175,9 @@ struct gpis_proposal {
     uint32_t cap = 0;
     std::vector<void *> act;
     bf *xb = nullptr, *ub = nullptr, *hb = nullptr, *y1 = nullptr, *y2 = nullptr, *y3 = nullptr, *dob = nullptr,
-       *dab = nullptr, *dgib = nullptr, *dghb = nullptr;
-    float *h = nullptr, *gi = nullptr, *gh = nullptr, *r = nullptr, *z = nullptr, *nn = nullptr, *ghn = nullptr,
+       *dab = nullptr;
+    // gates: the products of the input, then the gates, then the gates' gradients
+    float *h = nullptr, *gates = nullptr, *gh = nullptr, *ghn = nullptr,
           *a1 = nullptr, *a2 = nullptr, *a3 = nullptr, *o = nullptr, *dy = nullptr,
           *du = nullptr, *dh = nullptr, *loss = nullptr;
     // fused inference: GPIS_PROPOSAL_KERNEL_*, resident blocks per SM of each form, and
@@ -1215,16 +1225,14 @@ int ensure_batch(gpis_proposal *p, uint32_t n)
     PTRY(palloc(p, p->ub, N * MLPIN), "allocate proposal activations");
     PTRY(palloc(p, p->hb, N * (NHIST + 1) * HID), "allocate proposal activations");
     PTRY(palloc(p, p->h, N * (NHIST + 1) * HID), "allocate proposal activations");
-    PTRY(palloc(p, p->gi, N * NHIST * 3 * HID), "allocate proposal activations");
+    PTRY(palloc(p, p->gates, N * NHIST * 3 * HID), "allocate proposal activations");
     PTRY(palloc(p, p->gh, N * 3 * HID), "allocate proposal activations");
-    for (float **q : {&p->r, &p->z, &p->nn, &p->ghn}) PTRY(palloc(p, *q, N * NHIST * HID), "allocate proposal activations");
+    PTRY(palloc(p, p->ghn, N * NHIST * HID), "allocate proposal activations");
     for (float **q : {&p->a1, &p->a2, &p->a3, &p->dy}) PTRY(palloc(p, *q, N * WID), "allocate proposal activations");
     for (bf **q : {&p->y1, &p->y2, &p->y3, &p->dab}) PTRY(palloc(p, *q, N * WID), "allocate proposal activations");
     PTRY(palloc(p, p->o, N * NOUT), "allocate proposal activations");
     PTRY(palloc(p, p->dob, N * NOUT), "allocate proposal activations");
     PTRY(palloc(p, p->du, N * MLPIN), "allocate proposal activations");
-    PTRY(palloc(p, p->dgib, N * NHIST * 3 * HID), "allocate proposal activations");
-    PTRY(palloc(p, p->dghb, N * NHIST * 3 * HID), "allocate proposal activations");
     PTRY(palloc(p, p->dh, N * HID), "allocate proposal activations");
     PTRY(palloc(p, p->loss, 1), "allocate proposal activations");
     p->cap = n;
@@ -1255,13 +1263,13 @@ void forward(gpis_proposal *p, const float *feat, uint32_t n, cudaStream_t s)
     const bf *wb = p->pb;
     k_prep<<<dim3(nb(n, 128), NHIST + 2), 128, 0, s>>>(feat, n, p->xb, p->ub, p->h, p->hb);
     // the input products of every step at once
-    gemm(p, s, p->xb, NIN, 1, wb + O_WIH, 1, NIN, p->gi, 3 * HID, NHIST * n, 3 * HID, NIN, 0);
+    gemm(p, s, p->xb, NIN, 1, wb + O_WIH, 1, NIN, p->gates, 3 * HID, NHIST * n, 3 * HID, NIN, 0);
     for (int j = 0; j < NHIST; ++j) {
         const bf *hb = p->hb + (size_t)j * n * HID;
         gemm(p, s, hb, HID, 1, wb + O_WHH, 1, HID, p->gh, 3 * HID, n, 3 * HID, HID, 0);
         const size_t o = (size_t)j * n * HID;
-        k_gru_cell<<<nb((size_t)n * HID), 256, 0, s>>>(p->gi + (size_t)j * n * 3 * HID, p->gh, p->p, p->h + o, n, p->r + o, p->z + o, p->nn + o,
-                                                        p->ghn + o, p->h + o + (size_t)n * HID, p->hb + o + (size_t)n * HID,
+        k_gru_cell<<<nb((size_t)n * HID), 256, 0, s>>>(p->gates + 3 * o, p->gh, p->p, p->h + o, n, p->ghn + o,
+                                                        p->h + o + (size_t)n * HID, p->hb + o + (size_t)n * HID,
                                                         j == NHIST - 1 ? p->ub : nullptr);
     }
     gemm(p, s, p->ub, MLPIN, 1, wb + O_W1, 1, MLPIN, p->a1, WID, n, WID, MLPIN, 0);
@@ -1305,16 +1313,17 @@ void backward(gpis_proposal *p, const float2 *tgt, uint32_t n, cudaStream_t s)
     long ldh = MLPIN;
     for (int j = NHIST - 1; j >= 0; --j) {
         const size_t o = (size_t)j * n * HID;
-        bf *dgib = p->dgib + 3 * o, *dghb = p->dghb + 3 * o;
         k_gru_back<<<std::min(nb((size_t)n * HID), kBackBlocks), 256, 0, s>>>(
-            dh, ldh, p->r + o, p->z + o, p->nn + o, p->ghn + o, p->h + o, n, dgib, dghb, p->dh, G + O_BIH, G + O_BHH);
-        if (j > 0) gemm(p, s, dghb, 3 * HID, 1, wb + O_WHH, HID, 1, p->dh, HID, n, HID, 3 * HID, 1);
+            dh, ldh, p->gates + 3 * o, p->ghn + o, p->h + o, n, p->dh, G + O_BIH, G + O_BHH);
+        const bf *dghb = reinterpret_cast<const bf *>(p->gates + 3 * o) + 3 * HID;
+        if (j > 0) gemm(p, s, dghb, kGateRow, 1, wb + O_WHH, HID, 1, p->dh, HID, n, HID, 3 * HID, 1);
         dh = p->dh;
         ldh = HID;
     }
     const size_t rows = (size_t)NHIST * n;
-    gemm(p, s, p->dgib, 1, 3 * HID, p->xb, NIN, 1, G + O_WIH, NIN, 3 * HID, NIN, (int)rows, 1, ksplit_for(rows));
-    gemm(p, s, p->dghb, 1, 3 * HID, p->hb, HID, 1, G + O_WHH, HID, 3 * HID, HID, (int)rows, 1, ksplit_for(rows));
+    const bf *dg = reinterpret_cast<const bf *>(p->gates);
+    gemm(p, s, dg, 1, kGateRow, p->xb, NIN, 1, G + O_WIH, NIN, 3 * HID, NIN, (int)rows, 1, ksplit_for(rows));
+    gemm(p, s, dg + 3 * HID, 1, kGateRow, p->hb, HID, 1, G + O_WHH, HID, 3 * HID, HID, (int)rows, 1, ksplit_for(rows));
 }
 
 // Resident blocks per SM of a kernel with `dyn` bytes of dynamic shared memory (opted in
