@@ -5032,7 +5032,7 @@ __global__ void k_se_splat_1d(const float *q, const float *c, float *v, float *d
 
 }  // namespace
 
-cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream, cudaEvent_t *ev)
+cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream, cudaEvent_t *ev, uint64_t *kernels)
 {
     if (a.n == 0) return cudaSuccess;
     // one thread per flight; with a live count in device memory, grid-stride over a
@@ -5056,7 +5056,9 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
     // flight order instead (an uneven image batch 496 against 512 ms with a queue)
     const bool group3 = a.three_d && a.max_oct == 1 && !a.any_ns && !a.any_gen3d && a.max_imp <= (uint32_t)kG3Imp;
     if (!group1 && !group3) b.queue = nullptr;
+    uint64_t launched = 1;      // k_finish
     if (b.any_cond || b.setup) {
+        ++launched;
         if (a.one_d) k_prepare<8><<<blocks, 128, 0, stream>>>(b);
         else k_prepare<4><<<blocks, 128, 0, stream>>>(b);
     }
@@ -5064,8 +5066,9 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
     cudaError_t err = cudaMemsetAsync(b.work, 0, kWorkCounters * sizeof(uint32_t), stream);
     if (err != cudaSuccess) return err;
     // persistent grids: exactly the CTAs that are resident at once, never more
-    // warps than flights
+    // warps than flights (each march launch takes its grid here, once)
     auto grid = [&](const void *fn, size_t smem = 0, bool tuned = true, uint32_t group = 1) {
+        ++launched;
         const uint32_t ctas_needed = (uint32_t)(((uint64_t)a.n * group + 255) / 256);
         int per_sm = 0;
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, 256, smem) != cudaSuccess || per_sm < 1)
@@ -5222,6 +5225,7 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
     if (a.one_d) k_finish<8><<<blocks, 128, 0, stream>>>(b);
     else k_finish<4><<<blocks, 128, 0, stream>>>(b);
     if (ev) cudaEventRecord(ev[5], stream);
+    if (kernels) *kernels += launched;
     return cudaGetLastError();
 }
 

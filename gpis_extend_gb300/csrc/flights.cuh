@@ -97,7 +97,9 @@ cudaError_t upload_pcg_table();
 
 // Enqueue the flight kernels on the stream.  ev, when not null, holds start/stop
 // events for the prepare, march (march + resume) and finish kernels (ev[2k], ev[2k+1]).
-cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream, cudaEvent_t *ev = nullptr);
+// kernels: may be null; the number of kernels launched is added to it
+cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream, cudaEvent_t *ev = nullptr,
+                           uint64_t *kernels = nullptr);
 // Fill the corner table of a grid mean (m holds the device voxel pointer and cell_lo/cell_n)
 cudaError_t launch_pack_grid(const DevMedium &m, float4 *cells, size_t n, cudaStream_t stream);
 // 1D specular NEE queries on the realizations of the flights in a (one thread each)

@@ -282,6 +282,7 @@ struct gpis_ctx {
     std::vector<cudaEvent_t> ev_pending;   // groups of 6 recorded events
     double prof_ms[3] = {0, 0, 0};
     uint64_t prof_launches[3] = {0, 0, 0};
+    uint64_t launched = 0;                 // kernels launched by flight, feature and NEE batches
     // schedule knobs (gpis_tune_set; 0 = default)
     uint64_t tune[7] = {0, 0, 0, 0, 0, 0, 0};
 };
@@ -552,7 +553,7 @@ int submit_slice(gpis_ctx *ctx, const gpis_flight_soa *in, const gpis_result_soa
         }
         ev = evs;
     }
-    CUDA_TRY(gpis::launch_flights(a, ctx->num_sms, stream, ev), "launch flights");
+    CUDA_TRY(gpis::launch_flights(a, ctx->num_sms, stream, ev, &ctx->launched), "launch flights");
     if (ctx->profiling) {
         ctx->prof_launches[0] += a.any_cond ? 1 : 0;
         ctx->prof_launches[1] += 1;
@@ -612,8 +613,11 @@ __attribute__((visibility("hidden"))) int gpis_internal_features_live(gpis_ctx *
     CUDA_TRY(gpis::launch_features(ctx->d_media, ctx->n_media, *in, cap, features,
                                    static_cast<cudaStream_t>(cuda_stream), n_dev),
              "proposal features");
+    ctx->launched += 1;
     return GPIS_OK;
 }
+
+__attribute__((visibility("hidden"))) uint64_t gpis_internal_launched(gpis_ctx *ctx) { return ctx->launched; }
 
 __attribute__((visibility("hidden"))) int gpis_internal_nee_live(gpis_ctx *ctx, const gpis_nee_soa *in, float *out,
                                                                  uint32_t cap, const uint32_t *n_dev,
@@ -636,11 +640,10 @@ __attribute__((visibility("hidden"))) int gpis_internal_nee_live(gpis_ctx *ctx, 
                               reinterpret_cast<const float4 *>(in->normal), reinterpret_cast<float4 *>(out),
                               static_cast<cudaStream_t>(cuda_stream)),
              "launch NEE");
+    ctx->launched += 1;
     return GPIS_OK;
 }
 
-// SM count, whether per-kernel profiling is on, and whether a flight batch runs the
-// prepare kernel (conditioning media, or the 1D passes' set-up records)
 int gpis_tune_set(gpis_ctx *ctx, uint32_t key, uint64_t value)
 {
     if (!ctx) return fail(GPIS_EINVAL, "null context");
@@ -701,13 +704,12 @@ __attribute__((visibility("hidden"))) uint32_t gpis_internal_render_pass(gpis_ct
                                                          : (1u << 22);
 }
 
-__attribute__((visibility("hidden"))) int gpis_internal_ctx_info(gpis_ctx *ctx, int *num_sms, int *profiling,
-                                                                 int *prepare_runs)
+// SM count and whether per-kernel profiling is on
+__attribute__((visibility("hidden"))) int gpis_internal_ctx_info(gpis_ctx *ctx, int *num_sms, int *profiling)
 {
     if (!ctx) return GPIS_EINVAL;
     if (num_sms) *num_sms = ctx->num_sms;
     if (profiling) *profiling = ctx->profiling ? 1 : 0;
-    if (prepare_runs) *prepare_runs = (ctx->any_cond || ctx->setup_len) ? 1 : 0;
     return GPIS_OK;
 }
 

@@ -849,8 +849,9 @@ extern "C" int gpis_internal_infer_live(gpis_proposal *p, const gpis_flight_soa 
 extern "C" int gpis_internal_proposal_quiesce(gpis_proposal *p);
 extern "C" int gpis_internal_nee_live(gpis_ctx *ctx, const gpis_nee_soa *in, float *out, uint32_t cap,
                                       const uint32_t *n_dev, void *cuda_stream);
-extern "C" int gpis_internal_ctx_info(gpis_ctx *ctx, int *num_sms, int *profiling, int *prepare_runs);
+extern "C" int gpis_internal_ctx_info(gpis_ctx *ctx, int *num_sms, int *profiling);
 extern "C" uint32_t gpis_internal_render_pass(gpis_ctx *ctx);
+extern "C" uint64_t gpis_internal_launched(gpis_ctx *ctx);
 extern "C" int gpis_internal_render_block(gpis_ctx *ctx, size_t bytes, void **block);
 extern "C" void gpis_internal_render_done(gpis_ctx *ctx);
 
@@ -973,8 +974,8 @@ extern "C" int gpis_render_batch_proposed(gpis_ctx *ctx, gpis_proposal *prop, co
         cap = std::max(cap, pass_n[p]);
         max_segs = std::max<uint32_t>(max_segs, (uint32_t)passes[p].size());
     }
-    int num_sms = 1, profiling = 0, prepare_runs = 1;
-    gpis_internal_ctx_info(ctx, &num_sms, &profiling, &prepare_runs);
+    int num_sms = 1, profiling = 0;
+    gpis_internal_ctx_info(ctx, &num_sms, &profiling);
 
     RtScene *d_scenes;
     Seg *d_segs;
@@ -1068,16 +1069,23 @@ extern "C" int gpis_render_batch_proposed(gpis_ctx *ctx, gpis_proposal *prop, co
     }
     // the flight scratch for the largest batch, allocated before any capture (the
     // queue counters are zero here, so these launches trace nothing)
+    uint64_t n_launch = 0;
+    const uint64_t before = gpis_internal_launched(ctx);
     int rc = gpis_internal_submit_live(ctx, &sin, &sout, 2 * cap, counts + 1, st, nullptr);
     if (rc) return rc;
     if (any_nee) {
         rc = gpis_internal_nee_live(ctx, &nin, reinterpret_cast<float *>(eq.out), 2 * cap, counts + 2, st);
         if (rc) return rc;
     }
+    n_launch += gpis_internal_launched(ctx) - before;
     const unsigned tb = 128;
     const unsigned gs = (unsigned)std::max(1, num_sms * 8);   // grid of the grid-stride kernels
-    // one round of the bounce loop; every length it needs is in device memory
+    // one round of the bounce loop; every length it needs is in device memory.  `kernels`
+    // is the number it launches, the same in every round: of the flight batches' passes those
+    // too whose range the live count turns out to miss
+    uint64_t kernels = 0;
     auto round = [&]() -> int {
+        const uint64_t batches = gpis_internal_launched(ctx);
         cudaError_t e = cudaMemsetAsync(counts, 0, 3 * sizeof(uint32_t), st);
         if (e != cudaSuccess) return cuda_fail(e, "clear queue counters");
         k_rt_advance<<<gs, tb, 0, st>>>(d_scenes, paths, n_paths, q, dcnt);
@@ -1101,12 +1109,10 @@ extern "C" int gpis_render_batch_proposed(gpis_ctx *ctx, gpis_proposal *prop, co
         k_rt_shadow<<<gs, tb, 0, st>>>(sq, counts, direct);
         k_rt_collect<<<gs, tb, 0, st>>>(paths, q.path, counts, direct);
         k_rt_tally<<<1, 32, 0, st>>>(counts, dcnt);
+        // advance, event, shadow, collect, tally, the shading of NEE events and the inference
+        kernels = gpis_internal_launched(ctx) - batches + 5 + (any_nee ? 1 : 0) + (prop ? 1 : 0);
         return GPIS_OK;
     };
-    // kernels of one round: advance, event, shadow, collect, tally, and per flight batch
-    // prepare (when it runs), march, resume and finish; NEE adds its kernel and the shading
-    const uint64_t per_batch = 3 + (prepare_runs ? 1 : 0);
-    const uint64_t per_round = 5 + 2 * per_batch + (any_nee ? 2 : 0) + (prop ? 2 : 0);
     const uint32_t rounds = 2 * max_bounces + 4;
     cudaGraphExec_t gexec = nullptr;
     struct GraphGuard { cudaGraphExec_t g; ~GraphGuard() { if (g) cudaGraphExecDestroy(g); } } gg{nullptr};
@@ -1130,7 +1136,6 @@ extern "C" int gpis_render_batch_proposed(gpis_ctx *ctx, gpis_proposal *prop, co
     }
     if (stats) stats->graphed = graphed ? 1u : 0u;
     RT_TRY(cudaEventRecord(e0, st), "record event");
-    uint64_t n_launch = 0;
     for (size_t p = 0; p < passes.size(); ++p) {
         const std::vector<Seg> &segs = passes[p];
         RT_TRY(cudaMemcpyAsync(d_segs, segs.data(), segs.size() * sizeof(Seg), cudaMemcpyHostToDevice, st),
@@ -1145,7 +1150,7 @@ extern "C" int gpis_render_batch_proposed(gpis_ctx *ctx, gpis_proposal *prop, co
                 rc = round();
                 if (rc) return rc;
             }
-            n_launch += per_round;
+            n_launch += kernels;
         }
         k_rt_accumulate<<<(pass_pix[p] + tb - 1) / tb, tb, 0, st>>>(d_scenes, d_segs, (int)segs.size(), paths,
                                                                     pass_pix[p], acc);

@@ -460,8 +460,7 @@ typedef struct {
     uint64_t medium_events;
     uint64_t failed;            /* paths ended by a failed medium or phase sample */
     double ms;                  /* device time of the render (CUDA events)        */
-    uint64_t launches;          /* kernels launched by the render (the passes of a
-                                   flight batch counted as one march and one resume) */
+    uint64_t launches;          /* kernels launched by the render                 */
     uint64_t nee_queries;       /* neePDF / neeGrad queries of specular events    */
     uint32_t graphed;           /* 1: the bounce loop ran as a captured CUDA graph */
     uint32_t passes;            /* passes of up to 2^22 paths                     */
