@@ -2796,11 +2796,12 @@ struct LevelOrigin {
     float oz[2];
 };
 
+template <bool LEVELS = true>
 __device__ __forceinline__ FastPoint fast_point(const LaneField &L, float px, float py, float pz, LevelOrigin &lo)
 {
     const DevMedium &m = *L.m;
     FastPoint q;
-    q.mr = (m.flags & MF_MULTIRES) != 0;
+    q.mr = LEVELS && (m.flags & MF_MULTIRES) != 0;
     q.lv = {};
     q.oz[0] = q.oz[1] = 0.0f;
     q.ls = 1.0f;
@@ -3578,7 +3579,8 @@ struct EvalCoop1D {
 // 1D evaluator for media with several octaves, a nonstationary length scale or the
 // multi-resolution grid (whose two levels count as octaves here): each octave's
 // three-cell impulse window lives in shared memory, and the cells of all octaves are drawn
-// together (window_fill).  Every lane of the warp must call value().
+// together (window_fill).  NOCT: the most octaves (or levels) of the batch's media.  Every
+// lane of the warp must call value().
 //
 // What bounds it: issue slots and the instruction cache.  Drawing per octave and slot
 // (nine ballots and loops per evaluation), taking the skip bound's per-flight terms and
@@ -3586,6 +3588,7 @@ struct EvalCoop1D {
 // flight's set-up inside the march cost 2 540 instructions per lane and evaluation.
 constexpr int kOctMax = 4;
 
+template <int NOCT>
 struct EvalCoopOct {
     static constexpr bool kCollective = true;
     static constexpr int kGroup = 1;
@@ -3594,7 +3597,7 @@ struct EvalCoopOct {
     static constexpr bool kSkip = false;
     float *cbase;
     uint4 *list;
-    int base[kOctMax];
+    int base[NOCT];
     uint32_t rot;
     uint32_t valid;         // bit o: octave o's window is filled
     uint32_t level;         // multi-resolution: the lower level's seed offset of the windows
@@ -3614,7 +3617,7 @@ struct EvalCoopOct {
     __device__ __forceinline__ float value(const LaneField &L, float px, float py, float pz,
                                            int &id, uint32_t &refills, bool live)
     {
-        const FastPoint q = fast_point(L, px, py, pz, lo);
+        const FastPoint q = fast_point<(NOCT > 1)>(L, px, py, pz, lo);
         const int n_oct = live ? (q.mr ? 2 : (int)L.m->n_oct) : 0;
         last_ls = q.ls;
         if (q.mr && q.lv.seed[0] != level) {
@@ -3622,12 +3625,12 @@ struct EvalCoopOct {
             level = q.lv.seed[0];
         }
         const int warp_oct = __reduce_max_sync(FULL, (unsigned)n_oct);
-        float z[kOctMax], frac[kOctMax];
-        uint32_t seeds[kOctMax];
+        float z[NOCT], frac[NOCT];
+        uint32_t seeds[NOCT];
         uint32_t kinds = 0u;
         int count = 0;
 #pragma unroll
-        for (int o = 0; o < kOctMax; ++o) {
+        for (int o = 0; o < NOCT; ++o) {
             if (o >= warp_oct) break;
             const bool act = o < n_oct;
             seeds[o] = fast_seed(L, q, o);
@@ -3643,10 +3646,10 @@ struct EvalCoopOct {
             }
         }
         refills += (uint32_t)count;
-        window_fill<kOctMax>(list, cbase, sj, kinds, count, base, rot, seeds, L.n_imp);
+        window_fill<NOCT>(list, cbase, sj, kinds, count, base, rot, seeds, L.n_imp);
         float total = 0.0f;
 #pragma unroll
-        for (int o = 0; o < kOctMax; ++o) {
+        for (int o = 0; o < NOCT; ++o) {
             if (o >= warp_oct) break;
             if (o >= n_oct) continue;
             const int r = (rot >> (2 * o)) & 3u;
@@ -3835,7 +3838,7 @@ __device__ __forceinline__ float skip_scale(const DevMedium &m, float px, float 
 
 // the evaluators whose fast pass skips by oct_skip_count
 template <class E> struct IsOct { static constexpr bool value = false; };
-template <> struct IsOct<EvalCoopOct> { static constexpr bool value = true; };
+template <int NOCT> struct IsOct<EvalCoopOct<NOCT>> { static constexpr bool value = true; };
 template <> struct IsOct<EvalWarp1D<true>> { static constexpr bool value = true; };
 template <> struct IsOct<EvalGroup1D<false, true>> { static constexpr bool value = true; };
 
@@ -5154,10 +5157,21 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
         }, [&] {
             b.hand_over = plain ? (a.all_grid ? 0u : kHandOverPlain) : kHandOverGeneral;
             if (!plain) {
-                const void *fn = (const void *)k_march<EvalCoopOct, false>;
-                const size_t smem = smem_window(std::max<uint32_t>(a.max_oct, a.any_mr ? 2u : 1u));
-                failed = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_window(kOctMax));
-                k_march<EvalCoopOct, false><<<grid(fn, smem), 256, smem, stream>>>(b);
+                // the evaluator's octave loops at the batch's count (one for a nonstationary
+                // single octave, two also for the grid's levels): 1 048 576 flights of one
+                // octave 7.40 ms a batch, with loops to four 9.04; of two 14.3 / 15.6, 60 000
+                // on the grid 3.50 / 3.61
+                auto octaves = [&](auto count) {
+                    using Oct = EvalCoopOct<decltype(count)::value>;
+                    const void *fn = (const void *)k_march<Oct, false>;
+                    const size_t smem = smem_window(std::max<uint32_t>(a.max_oct, a.any_mr ? 2u : 1u));
+                    failed = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                  (int)smem_window(decltype(count)::value));
+                    k_march<Oct, false><<<grid(fn, smem), 256, smem, stream>>>(b);
+                };
+                if (a.max_oct == 1u && !a.any_mr) octaves(std::integral_constant<int, 1>());
+                else if (a.max_oct <= 2u) octaves(std::integral_constant<int, 2>());
+                else octaves(std::integral_constant<int, kOctMax>());
             } else if (a.all_grid) {
                 using Grid = EvalCoop1D<8, true, true>;
                 const void *fn = (const void *)k_march<Grid, false>;
