@@ -85,6 +85,7 @@ struct DevMedium {
     float skip_mean_lip;
     float skip_noise_lip;   // 3 N e^{-1/2} / norm1d per iso unit
     float skip_jump;        // e^{-kr^2/2} / norm1d per truncation crossing
+    float skip_ls_slope;    // the local scale's largest change per unit of lateral travel (0: constant)
     float oct_inv[4];       // 1 / oct_scale[k], exact where the scale is a power of two
     uint32_t oct_pow2;      // bit k: oct_scale[k] is a power of two (x / s == x * oct_inv[k])
     // multi-resolution grid (MF_MULTIRES; ls_kind is 0 on the device so that the

@@ -1002,12 +1002,18 @@ __device__ __forceinline__ CondRec make_condition(const DevMedium &m, const Flig
 // ---------------------------------------------------------------------------
 // Per-flight set-up of the march over 1D media, computed here with every lane busy
 // instead of inside the march, where it runs for the few lanes that start a flight
-// while the rest of the warp waits.  Stationary single-octave media, four float4 per
-// flight: {frame normal, origin coordinate}, {value scale, gradient scale, step, t0},
-// {the four of reach_params}, {seed, flags, -, -}.  Other 1D media,
-// eight: {frame normal, scale at the origin}, {step, t0, seed, flags}, two of skip
-// constants (skip_consts), then value scales, gradient scales along the ray and origin
-// coordinates of up to four octaves, {the origin's level weights, -, -}.
+// while the rest of the warp waits: kSetupLen float4 per flight.  Stationary single-octave
+// media: {frame normal, origin coordinate}, {value scale, gradient scale, step, t0}, {the
+// four of reach_params}, {seed, flags, -, -}.  Other 1D media: {frame normal, scale at the
+// origin}, {step (negative: not a valid flight), t0, two of skip_consts' sums}, {the other
+// four; the first three's signs are the flags direct, conditioned and first scatter}, {the octaves' origin coordinates, or the origin's two level weights}; what is a
+// few operations from the streams, the medium or the conditioning record is taken again at
+// the flight's start, so that a batch needs no more scratch than a plain one.
+__device__ __forceinline__ float with_flag(float v, bool flag)
+{
+    return __uint_as_float(__float_as_uint(v) | (flag ? 0x80000000u : 0u));
+}
+__device__ __forceinline__ bool has_flag(float v) { return (__float_as_uint(v) & 0x80000000u) != 0u; }
 enum : uint32_t { SF_VALID = 1u, SF_COND = 2u, SF_FIRST = 4u, SF_DIRECT = 8u };
 __device__ __forceinline__ bool t_direct_ok(float t0, float step, float far_t);
 
@@ -1077,6 +1083,12 @@ __device__ __forceinline__ void reach_params(const DevMedium &m, const FlightIn 
     if (m.skip_mean_lip < 0.0f) curv = -1.0f;
 }
 
+// The gradient scale of octave k along the ray times the octave's length multiplier.
+__device__ __forceinline__ float cond_slope(const DevMedium &m, const CondRec &c, int k)
+{
+    return m.n_oct == 1 ? c.oct[k].gs[2] : __fmul_rn(oct_scale(m, k), c.oct[k].gs[2]);
+}
+
 // A conditioned 1D flight's coefficients per octave as the evaluators take them: value
 // scale, gradient scale along the ray times the octave's length multiplier, and the
 // origin's ray coordinate.
@@ -1087,31 +1099,32 @@ __device__ __forceinline__ void cond_1d(const DevMedium &m, const CondRec &c, co
         if (k >= (int)m.n_oct) break;
         const float sc = oct_scale(m, k);
         vs[k] = c.oct[k].vs;
-        gz[k] = m.n_oct == 1 ? c.oct[k].gs[2] : __fmul_rn(sc, c.oct[k].gs[2]);
+        gz[k] = cond_slope(m, c, k);
         oz[k] = ray_coord_oct(m, n, o[0], o[1], o[2], sc);
     }
 }
 
 // What oct_skip_count needs of a flight beyond the local scale: {mean slope, largest
-// change of the local scale per unit of t, sum of |amplitude|, and of |amplitude| times
-// the octave's iso units per unit of t; the same two sums with |value scale| and
-// |gradient scale|: (vs dz, gz dz, vs, gz)}.
+// change of the local scale per unit of t (skip_slopes), sum of |amplitude|, and of
+// |amplitude| times the octave's iso units per unit of t; the same two sums with |value
+// scale| and |gradient scale|: (vs dz, gz dz, vs, gz)}.
+__device__ __forceinline__ void skip_slopes(const DevMedium &m, const float d[3], float sk[8])
+{
+    // (a valid direction is of unit length within 5e-4)
+    sk[0] = m.skip_mean_lip * 1.0006f;
+    sk[1] = m.skip_ls_slope;
+    if (sk[1] != 0.0f) sk[1] *= sqrtf(d[0] * d[0] + d[2] * d[2]);
+}
+
 __device__ __forceinline__ void skip_consts(const DevMedium &m, const float d[3], bool cond, const float vs[4],
                                             const float gz[4], float sk[8])
 {
+    skip_slopes(m, d, sk);
 #pragma unroll
-    for (int k = 0; k < 8; ++k) sk[k] = 0.0f;
+    for (int k = 2; k < 8; ++k) sk[k] = 0.0f;
     const float lx = m.l_inv[0] * d[0], ly = m.l_inv[1] * d[1], lz = m.l_inv[2] * d[2];
     float dn = sqrtf(lx * lx + ly * ly + lz * lz) * 1.0001f;
-    sk[0] = m.skip_mean_lip * sqrtf(d[0] * d[0] + d[1] * d[1] + d[2] * d[2]);
-    if (m.ls_kind || (m.flags & MF_MULTIRES)) {
-        const float *q = m.ls_params;
-        sk[1] = fabsf(q[1]) * sqrtf(q[2] * q[2] + q[3] * q[3]) * sqrtf(d[0] * d[0] + d[2] * d[2]) * 1.0001f;
-    }
-    if (m.ls_kind) {
-        sk[1] /= m.ls_max;
-        dn /= m.ls_max;
-    }
+    if (m.ls_kind) dn /= m.ls_max;
 #pragma unroll
     for (int k = 0; k < 4; ++k) {
         if (k >= (int)m.n_oct) break;
@@ -1149,10 +1162,10 @@ __device__ __forceinline__ void prepare_one(const FlightArgs &a, uint32_t i)
         }
     }
     if (!a.setup) return;
-    const bool general = a.setup_len == 8u;
-    float4 *s = a.setup + (size_t)a.setup_len * i;
+    const bool general = a.setup_general != 0u;
+    float4 *s = a.setup + (size_t)kSetupLen * i;
     if (!valid || !(m.flags & MF_ONE_D)) {
-        if (general) s[1] = make_float4(0.0f, 0.0f, 0.0f, __uint_as_float(0u));
+        if (general) s[1] = make_float4(-1.0f, 0.0f, 0.0f, 0.0f);
         else s[3] = make_float4(0.0f, __uint_as_float(0u), 0.0f, 0.0f);
         return;
     }
@@ -1161,28 +1174,25 @@ __device__ __forceinline__ void prepare_one(const FlightArgs &a, uint32_t i)
     float step = __fdiv_rn(__fsub_rn(fl.far_t, fl.near_t), (float)m.min_step);
     if (m.step_size < step) step = m.step_size;
     const float t0 = __fadd_rn(fl.near_t, __fmul_rn(step, fl.jitter));
-    const uint32_t flags = SF_VALID | (cond ? SF_COND : 0u) | ((fl.flags & GPIS_FLAG_FIRST_SCATTER) ? SF_FIRST : 0u) |
-                           (t_direct_ok(t0, step, fl.far_t) ? SF_DIRECT : 0u);
     if (general) {
         float vs[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gz[4] = {0.0f, 0.0f, 0.0f, 0.0f}, oz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
         float ls_o = 1.0f;
         if (cond) {
             ls_o = ns_scale_precise(m, fl.o[0], fl.o[2]);
             cond_1d(m, c, f.n, fl.o, vs, gz, oz);
-            s[4] = make_float4(vs[0], vs[1], vs[2], vs[3]);
-            s[5] = make_float4(gz[0], gz[1], gz[2], gz[3]);
-            s[6] = make_float4(oz[0], oz[1], oz[2], oz[3]);
             if (m.flags & MF_MULTIRES) {
                 const MrLevels lo = mr_levels(m, ls_value_precise(m, fl.o[0], fl.o[2]));
-                s[7] = make_float4(lo.w[0], lo.w[1], 0.0f, 0.0f);
+                s[3] = make_float4(lo.w[0], lo.w[1], 0.0f, 0.0f);
+            } else {
+                s[3] = make_float4(oz[0], oz[1], oz[2], oz[3]);
             }
         }
         float sk[8];
         skip_consts(m, fl.d, cond, vs, gz, sk);
         s[0] = make_float4(f.n[0], f.n[1], f.n[2], ls_o);
-        s[1] = make_float4(step, t0, __uint_as_float(fl.noise_seed), __uint_as_float(flags));
-        s[2] = make_float4(sk[0], sk[1], sk[2], sk[3]);
-        s[3] = make_float4(sk[4], sk[5], sk[6], sk[7]);
+        const bool first = (fl.flags & GPIS_FLAG_FIRST_SCATTER) != 0;
+        s[1] = make_float4(step, t0, with_flag(sk[2], t_direct_ok(t0, step, fl.far_t)), with_flag(sk[3], cond));
+        s[2] = make_float4(with_flag(sk[4], first), sk[5], sk[6], sk[7]);
         return;
     }
     const float ozc = cond ? ray_coord_oct(m, f.n, fl.o[0], fl.o[1], fl.o[2], 1.0f) : 0.0f;
@@ -1192,6 +1202,8 @@ __device__ __forceinline__ void prepare_one(const FlightArgs &a, uint32_t i)
     s[0] = make_float4(f.n[0], f.n[1], f.n[2], ozc);
     s[1] = make_float4(vs, gsz, step, t0);
     s[2] = make_float4(curv, j0, j1, dn);
+    const uint32_t flags = SF_VALID | (cond ? SF_COND : 0u) | ((fl.flags & GPIS_FLAG_FIRST_SCATTER) ? SF_FIRST : 0u) |
+                           (t_direct_ok(t0, step, fl.far_t) ? SF_DIRECT : 0u);
     s[3] = make_float4(__uint_as_float(fl.noise_seed), __uint_as_float(flags), 0.0f, 0.0f);
 }
 
@@ -1346,26 +1358,25 @@ __device__ __forceinline__ void lane_field_setup(LaneField &L, const DevMedium &
     }
 }
 
-// A lane's registers from the set-up record of its flight (LEN float4), its origin and
-// direction streams; false where the record says that the flight is not valid.
+// A lane's registers from the set-up record of flight idx; false where the record says that
+// the flight is not valid.  GENERAL: the record of octave, nonstationary and
+// multi-resolution media.
 struct LaneStart {
     float step, t0, curv, j0, j1, dn;
     bool first, direct;
 };
-template <int LEN>
-__device__ __forceinline__ bool lane_field_load(LaneField &L, const DevMedium &m, const float4 *s, const float4 &on,
-                                                LaneStart &st)
+template <bool GENERAL>
+__device__ __forceinline__ bool lane_field_load(LaneField &L, const DevMedium &m, const FlightArgs &a, uint32_t idx,
+                                                const float4 &on, const float4 &df, LaneStart &st)
 {
-    const float4 a = s[0], b = s[1], c = s[2], e = s[3];
-    const uint32_t flags = __float_as_uint(LEN == 8 ? b.w : e.y);
-    if (!(flags & SF_VALID)) return false;
-    st.first = (flags & SF_FIRST) != 0;
-    st.direct = (flags & SF_DIRECT) != 0;
+    const float4 *s = a.setup + (size_t)kSetupLen * idx;
+    const float4 s0 = s[0], s1 = s[1], s2 = s[2], s3 = s[3];
+    const uint32_t flags = __float_as_uint(s3.y);
+    if (GENERAL ? s1.x < 0.0f : !(flags & SF_VALID)) return false;
 #pragma unroll
     for (int k = 0; k < 3; ++k) L.li[k] = m.l_inv[k];
     L.o[0] = on.x; L.o[1] = on.y; L.o[2] = on.z;
-    L.n[0] = a.x; L.n[1] = a.y; L.n[2] = a.z;
-    L.cond = (flags & SF_COND) != 0;
+    L.n[0] = s0.x; L.n[1] = s0.y; L.n[2] = s0.z;
     L.sigma = m.sigma;
     L.mean_kind = m.mean_kind;
 #pragma unroll
@@ -1374,37 +1385,51 @@ __device__ __forceinline__ bool lane_field_load(LaneField &L, const DevMedium &m
     L.kr = m.kr_iso;
     L.kexp = m.kexp1d;
     L.inv_norm = m.inv_norm1d;
-    L.ns = LEN == 8 && m.ls_kind != 0u;
+    L.ns = GENERAL && m.ls_kind != 0u;
     L.mr_ow[0] = L.mr_ow[1] = 1.0f;
-    if (LEN == 8) {
-        L.ls_o = a.w;
-        L.seed = __float_as_uint(b.z);
-        st.step = b.x;
-        st.t0 = b.y;
-        L.sk[0] = c.x; L.sk[1] = c.y; L.sk[2] = c.z; L.sk[3] = c.w;
-        L.sk[4] = e.x; L.sk[5] = e.y; L.sk[6] = e.z; L.sk[7] = e.w;
+    if (GENERAL) {
+        const float d[3] = {df.x, df.y, df.z};
+        st.first = has_flag(s2.x);
+        st.step = s1.x;
+        st.t0 = s1.y;
+        st.direct = has_flag(s1.z);
+        L.cond = has_flag(s1.w);
+        L.seed = a.seeds[idx].x;
+        L.ls_o = s0.w;
+        skip_slopes(m, d, L.sk);
+        L.sk[2] = fabsf(s1.z); L.sk[3] = fabsf(s1.w);
+        L.sk[4] = fabsf(s2.x); L.sk[5] = s2.y; L.sk[6] = s2.z; L.sk[7] = s2.w;
         if (L.cond) {
-            const float4 v = s[4], g = s[5], z = s[6];
-            const float vs[4] = {v.x, v.y, v.z, v.w}, gz[4] = {g.x, g.y, g.z, g.w}, oz[4] = {z.x, z.y, z.z, z.w};
+            const CondRec &c = a.cond[idx];
+            float vs[4] = {0.0f, 0.0f, 0.0f, 0.0f}, gz[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+            const float oz[4] = {s3.x, s3.y, s3.z, s3.w};
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                if (k >= (int)m.n_oct) break;
+                vs[k] = c.oct[k].vs;
+                gz[k] = cond_slope(m, c, k);
+            }
             lane_cond_set(L, vs, gz, oz);
             if (m.flags & MF_MULTIRES) {
-                const float4 w = s[7];
-                L.mr_ow[0] = w.x;
-                L.mr_ow[1] = w.y;
+                L.mr_ow[0] = s3.x;
+                L.mr_ow[1] = s3.y;
             }
         }
     } else {
+        st.first = (flags & SF_FIRST) != 0;
+        st.direct = (flags & SF_DIRECT) != 0;
+        L.cond = (flags & SF_COND) != 0;
         L.ls_o = 1.0f;
-        L.ozc = a.w;
-        L.vs = b.x;
-        L.gsz = b.y;
-        st.step = b.z;
-        st.t0 = b.w;
-        st.curv = c.x;
-        st.j0 = c.y;
-        st.j1 = c.z;
-        st.dn = c.w;
-        L.seed = __float_as_uint(e.x);
+        L.ozc = s0.w;
+        L.vs = s1.x;
+        L.gsz = s1.y;
+        st.step = s1.z;
+        st.t0 = s1.w;
+        st.curv = s2.x;
+        st.j0 = s2.y;
+        st.j1 = s2.z;
+        st.dn = s2.w;
+        L.seed = __float_as_uint(s3.x);
     }
     return true;
 }
@@ -2920,7 +2945,7 @@ struct EvalGroup1D {
     static constexpr bool kCollective = false;
     static constexpr int kGroup = 8;
     static constexpr int kMinBlocks = 2;
-    static constexpr int kSetup = STAT ? 4 : 8;
+    static constexpr int kSetup = STAT ? 1 : 2;
     static constexpr bool kSkip = STAT;
     static constexpr int kThreads = 256;
     static constexpr int kWin = STAT ? 1 : 4;
@@ -3191,7 +3216,7 @@ struct EvalWarp1D {
     static constexpr bool kCollective = false;
     static constexpr int kGroup = 32;
     static constexpr int kMinBlocks = 2;
-    static constexpr int kSetup = 8;
+    static constexpr int kSetup = 2;
     static constexpr bool kSkip = false;
     EvalGroup1D<true, FAST> part;       // the octave's eight lanes: one window
     float last_ls;
@@ -3383,7 +3408,7 @@ struct EvalCoop1D {
     // CTAs per SM: with the window in shared memory 3 (80 registers), in registers 4 (64); a
     // grid mean's eight voxels want 2 (128; 500 009 flights 1.40 ms a batch, 1.75 with 3)
     static constexpr int kMinBlocks = GRID ? 2 : (SM ? 3 : 4);
-    static constexpr int kSetup = 4;
+    static constexpr int kSetup = 1;
     static constexpr bool kSkip = true;
     float cache[SM ? 1 : 3][SM ? 1 : NMAX];
     int base[1];
@@ -3593,7 +3618,7 @@ struct EvalCoopOct {
     static constexpr bool kCollective = true;
     static constexpr int kGroup = 1;
     static constexpr int kMinBlocks = 2;
-    static constexpr int kSetup = 8;
+    static constexpr int kSetup = 2;
     static constexpr bool kSkip = false;
     float *cbase;
     uint4 *list;
@@ -3960,8 +3985,9 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
     const uint32_t one = lead ? 1u : 0u;
     // single lanes pull flights when so many are idle: the pull's dependent loads and set-up
     // hold the whole warp (4.2 M sphere flights 6.17 ms pulling at once, 6.04 at 2, 5.79 at
-    // 4, 5.66 at 8 and at 12)
-    constexpr int kPull = G == 1 && Eval::kSetup == 4 ? 8 : 1;
+    // 4, 5.66 at 8 and at 12; general media, whose evaluations idle lanes hold up longer:
+    // 961 182 on the multi-resolution grid 17.3 at once, 16.9 at 4)
+    constexpr int kPull = G > 1 || Eval::kSetup == 0 ? 1 : (Eval::kSetup == 1 ? 8 : 4);
     constexpr bool kOwn3D = G > 1 && IsSkip3D<Eval>::value;     // marches on with its own evaluator
     uint32_t *work = a.work + (TAIL ? kWorkTail : (RESUME ? (CERT ? 1 : 2) : 0));
     const unsigned lt_mask = (1u << (lane & ~(G - 1))) - 1u;
@@ -4055,7 +4081,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                             // the set-up k_prepare computed for this flight
                             const float4 on = a.origin_near[idx], df = a.dir_far[idx];
                             LaneStart st = {};
-                            ok = mok && lane_field_load<Eval::kSetup>(L, m, a.setup + (size_t)Eval::kSetup * idx, on, st);
+                            ok = mok && lane_field_load<Eval::kSetup == 2>(L, m, a, idx, on, df, st);
                             d[0] = df.x; d[1] = df.y; d[2] = df.z;
                             near_t = on.w;
                             far_t = df.w;
@@ -5075,13 +5101,13 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
     FlightArgs b = a;
     // 1D media of up to 8 impulses per cell: the march passes take their per-flight set-up
     // from k_prepare; plain: every medium stationary with one octave
-    b.setup_len = setup_len(a.one_d, a.max_imp, a.max_oct, a.any_ns, a.any_mr);
-    const bool group1 = b.setup_len != 0u, plain = b.setup_len == 4u;
+    const bool group1 = takes_setup(a.one_d, a.max_imp), plain = a.max_oct == 1u && !a.any_ns && !a.any_mr;
+    b.setup_general = plain ? 0u : 1u;
     b.hand_over = 0u;
     b.run_lo = 0;
     b.run_hi = 0xffffffffu;
     if (!group1) b.setup = nullptr;     // the march kernels read set-up records only when written
-    const bool certify = plain && !a.all_grid && !a.precise_only;
+    const bool certify = group1 && plain && !a.all_grid && !a.precise_only;
     // stationary 3D media of up to 8 impulses per cell: lane groups, each of which loads
     // its flight's record once for all its lanes, so a queue's scattered order costs
     // nothing.  The one-lane evaluators of the other media scan every resume record in

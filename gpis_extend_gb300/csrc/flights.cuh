@@ -50,8 +50,8 @@ struct FlightArgs {
                                 // those the certified resume pass hands on (before it runs, those
                                 // that wait for the fast pass's tail)
     int queue_in;               // set by launch_flights for each resume pass
-    uint32_t setup_len;         // set by launch_flights: float4 per set-up record
-    float4 *setup;              // scratch, setup_len() per flight: the march passes' per-flight set-up,
+    uint32_t setup_general;     // set by launch_flights: 1 the set-up record of other than plain 1D media
+    float4 *setup;              // scratch, kSetupLen per flight: the march passes' per-flight set-up,
                                 // written by k_prepare for batches of 1D media (else unused)
     unsigned long long *counters;  // gpis_counters block (8 x u64)
     int any_cond;               // some medium conditions (run the prepare kernel)
@@ -80,13 +80,10 @@ struct FlightArgs {
 };
 
 // Batches of 1D media with up to 8 impulses per cell take the cooperative and lane-group
-// evaluators, whose flights start from the set-up record that k_prepare wrote: 4 float4
-// where every medium is stationary with one octave, 8 otherwise; 0: no record.
-inline uint32_t setup_len(bool one_d, uint32_t max_imp, uint32_t max_oct, bool any_ns, bool any_mr)
-{
-    if (!one_d || max_imp > 8u) return 0u;
-    return max_oct == 1u && !any_ns && !any_mr ? 4u : 8u;
-}
+// evaluators, whose flights start from the set-up record (kSetupLen float4) that k_prepare
+// wrote.
+constexpr uint32_t kSetupLen = 4;
+inline bool takes_setup(bool one_d, uint32_t max_imp) { return one_d && max_imp <= 8u; }
 
 // Per-flight features of the learned proposal (proposal.cu).
 cudaError_t launch_features(const DevMedium *media, int n_media, const gpis_flight_soa &in, uint32_t n, float *feat,

@@ -229,6 +229,11 @@ int derive_medium(const gpis_medium_desc &d, gpis::DevMedium &m)
     }
     m.skip_noise_lip = (float)(3.0 * m.n_imp * std::exp(-0.5) / (double)m.norm1d);
     m.skip_jump = (float)(std::exp(-0.5 * (double)m.kr_iso * m.kr_iso) / (double)m.norm1d);
+    m.skip_ls_slope = 0.0f;
+    if (d.ls_kind != GPIS_LS_CONSTANT)
+        m.skip_ls_slope = (float)(std::fabs((double)d.ls_params[1]) *
+                                  std::hypot((double)d.ls_params[2], (double)d.ls_params[3]) * 1.0001 /
+                                  (multires ? 1.0 : (double)d.ls_max));
     m.step_size = d.step_size;
     m.min_step = d.min_step;
     m.max_steps = d.max_steps ? d.max_steps : 16384u;
@@ -260,7 +265,7 @@ struct gpis_ctx {
     double *d_tend = nullptr;
     uint4 *d_resume = nullptr;
     float4 *d_setup = nullptr;
-    uint32_t setup_len = 0;                // float4 per flight of d_setup (gpis::setup_len)
+    bool setup = false;                    // batches take set-up records (gpis::takes_setup)
     uint32_t *d_queue = nullptr;
     uint32_t *d_work = nullptr;
     unsigned long long *d_counters = nullptr;
@@ -343,8 +348,8 @@ int ensure_scratch(gpis_ctx *c, size_t n)
     CUDA_TRY(cudaMalloc(&c->d_cond, cap * sizeof(gpis::CondRec)), "allocate conditioning scratch");
     CUDA_TRY(cudaMalloc(&c->d_tend, cap * sizeof(double)), "allocate end-parameter scratch");
     CUDA_TRY(cudaMalloc(&c->d_resume, cap * sizeof(uint4)), "allocate resume scratch");
-    if (c->setup_len)
-        CUDA_TRY(cudaMalloc(&c->d_setup, cap * c->setup_len * sizeof(float4)), "allocate set-up scratch");
+    if (c->setup)
+        CUDA_TRY(cudaMalloc(&c->d_setup, cap * gpis::kSetupLen * sizeof(float4)), "allocate set-up scratch");
     CUDA_TRY(cudaMalloc(&c->d_queue, cap * 2 * sizeof(uint32_t)), "allocate hand-off queues");
     c->cap = cap;
     return GPIS_OK;
@@ -464,7 +469,7 @@ int gpis_ctx_create(const gpis_medium_desc *media, int n_media, gpis_ctx **out)
             c->any_mr = c->any_mr || (m.flags & gpis::MF_MULTIRES) != 0u;
             c->any_gen3d = c->any_gen3d || gpis::general_3d(m);
         }
-        c->setup_len = gpis::setup_len(c->all_one_d, c->max_imp, c->max_oct, c->any_ns, c->any_mr);
+        c->setup = gpis::takes_setup(c->all_one_d, c->max_imp);
         if (rc) break;
         if ((e = cudaMalloc(&c->d_media, host.size() * sizeof(gpis::DevMedium))) != cudaSuccess) { rc = cuda_fail(e, "allocate media"); break; }
         if ((e = cudaMemcpy(c->d_media, host.data(), host.size() * sizeof(gpis::DevMedium), cudaMemcpyHostToDevice)) != cudaSuccess) {
@@ -522,7 +527,7 @@ int submit_slice(gpis_ctx *ctx, const gpis_flight_soa *in, const gpis_result_soa
     a.t_end = ctx->d_tend + offset;
     a.work = work;
     a.resume = ctx->d_resume + offset;
-    a.setup = ctx->d_setup + (size_t)ctx->setup_len * offset;
+    a.setup = ctx->setup ? ctx->d_setup + (size_t)gpis::kSetupLen * offset : nullptr;
     a.queue = ctx->d_queue + 2 * offset;
     a.counters = ctx->d_counters;
     a.any_cond = ctx->any_cond;

@@ -37,7 +37,7 @@ constexpr size_t kOffCond = kOffCounters + 256;
 constexpr size_t kOffTEnd = kOffCond + kMax * sizeof(gpis::CondRec);
 constexpr size_t kOffResume = kOffTEnd + kMax * sizeof(double);
 constexpr size_t kOffSetup = kOffResume + kMax * sizeof(uint4);
-constexpr size_t kOffQueue = kOffSetup + kMax * 8 * sizeof(float4);   // gpis::setup_len is at most 8
+constexpr size_t kOffQueue = kOffSetup + kMax * gpis::kSetupLen * sizeof(float4);
 constexpr size_t kBytes = kOffQueue + kMax * 2 * sizeof(uint32_t);
 static_assert(sizeof(gpis::DevMedium) <= kOffWork, "medium table must fit its slot");
 static_assert(gpis::kWorkCounters * sizeof(uint32_t) <= kOffCounters - kOffWork, "work counters must fit their slot");
