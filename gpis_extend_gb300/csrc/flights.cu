@@ -132,9 +132,9 @@ struct MrLevels {
     uint32_t seed[2];
 };
 
-// Float-float with a test of the rounding, the double evaluation for the values it cannot
-// decide; out of line, so that the march kernels of media without levels carry none of it
-// (three octaves, 300 007 flights: 9.05 ms a batch with it inline).
+// The two level weights at ls's place between the levels, as their double evaluation rounds:
+// float-float with a test of the rounding, the double evaluation for the values it cannot
+// decide.
 __device__ __forceinline__ float2 level_weights(float frac)
 {
     float w0, w1;
@@ -2815,7 +2815,6 @@ __device__ __forceinline__ T pick2(const T (&v)[2], int o) { return o & 1 ? v[1]
 // They have the reference's bits: a coordinate of the same size is subtracted, 10^4 where a
 // scene lies a thousand units from the origin, and there the level-free coordinate divided
 // by the scale, an ulp or two off, decided 0.8 % of short conditioned flights wrongly.
-// In shared memory: in registers they made the kernels spill for media without levels too.
 struct LevelOrigin {
     float s;                        // the lower level's scale (0: none)
     float oz[2];
@@ -2918,12 +2917,13 @@ __device__ __forceinline__ float fast_share(const LaneField &L, const FastPoint 
 // Batch times with group / single-lane resume passes (us): sphere field, precise pass,
 // 20 000 flights 364 / 452, 65 537 493 / 652, 262 144 979 / 1 172, 1 048 576 2 842 / 2 837;
 // its certified pass, 65 537 493 / 537, 262 144 979 / 950, 4 194 304 10 244 / 8 041; three
-// octaves, 30 000 flights 6 270 / 7 988, 300 007 15 288 / 16 116.  A group repeats the state
+// octaves, 30 000 flights 6 270 / 7 988.  A group repeats the state
 // machine and the coordinates in eight lanes, so long queues, which fill the chip with
 // single lanes, take those: about 0.55 of the flights cross, a fifth of these stay
 // uncertified, and the lines lie between the measured sizes where the two cross.
-// (Several octaves since the set-up records: 300 007 flights 9 503 / 10 935, 60 013 on the
-// multi-resolution grid 4 392 / 5 818.)
+// Precise pass of general media: three octaves, 300 007 flights 9 503 / 10 935, 1.2 M 25 476 /
+// 22 404, 4.2 M 83 303 / 72 322; a nonstationary octave, 1.2 M 8 771 / 7 179; multi-resolution,
+// 60 013 4 392 / 5 818, 1.2 M 21 543 / 20 144.
 constexpr uint32_t kFewCertified = 100000, kFewPrecise = 200000, kFewPreciseGeneral = 1000000;
 // Fast passes the same way, groups / lanes with their tail on groups: plain media, 10 000
 // flights 251 / 298, 20 000 242 / 268, 40 000 357 / 345, 65 537 425 / 338; three octaves,
@@ -3209,7 +3209,8 @@ struct EvalGroup1D {
 // Fast pass, warps / eights (us a batch): three octaves, 1 000 flights 1 400 / 2 379, 10 000
 // 2 328 / 2 999, 20 000 3 355 / 3 483, 40 000 5 800 / 4 732; multi-resolution, 3 000 1 439 /
 // 1 949, 10 000 2 207 / 2 198, 30 000 4 774 / 3 658.  Precise pass: three octaves, 10 000
-// 2 863 / 2 999, 100 000 5 416 / 5 676, 300 007 10 229 / 9 489.
+// 2 863 / 2 999, 80 000 4 186 / 4 127, 150 000 5 834 / 5 672, 300 007 10 229 / 9 489; a
+// nonstationary octave, 80 000 2 583 / 2 386; multi-resolution, 80 000 3 725 / 3 548.
 constexpr uint32_t kFewWarps = 12000, kFewWarpsPrecise = 60000;
 template <bool FAST>
 struct EvalWarp1D {
@@ -3721,11 +3722,11 @@ constexpr int kMaxSkip = 16;
 // inside the query's cell)
 constexpr int kMaxSkip3D = 32;
 
-// Step skipping for multi-octave and nonstationary 1D media (EvalCoopOct, and
-// EvalCoop1D's nonstationary form): a Lipschitz bound along the ray over the next
-// `cap` steps, from the local scale's range there (multi-octave evaluations cost
-// more than the warp's skip loop, so they may skip 16 steps; single-octave ones 8).  Octave k's noise is A(ls) S_k + C_k with S_k the sum of at
-// most 3N truncated splats exp(-(z_k - z_i)^2 / (2 ls^2)) in the octave's iso
+// Step skipping for multi-octave, nonstationary and multi-resolution 1D media (EvalCoopOct,
+// EvalGroup1D and EvalWarp1D): a Lipschitz bound along the ray over the `cap` steps on
+// either side, from the local scale's range there (the caller's span follows the last
+// reach, up to kMaxReach).  Octave k's noise is A(ls) S_k + C_k with S_k the sum of at most
+// 3N truncated splats exp(-(z_k - z_i)^2 / (2 ls^2)) in the octave's iso
 // coordinate z_k (|dz_k/dt| <= |l_inv o d| / (ls_max sc_k)), A(ls) = inv_norm1d
 // ls^-1/2 the normalisation and C_k the conditioning splats.  Per splat |dK/dz| <=
 // e^-1/2 / ls and |dK/dls| <= 2 / (e ls); |S_k| <= 3N; |dA/dls| = A / (2 ls); the
@@ -3736,8 +3737,8 @@ constexpr int kMaxSkip3D = 32;
 // q3^2) / ls_max per unit of lateral (x, z) travel.  Every bound takes the worst
 // local scale of the range.  A splat jumps by at most exp(-kr^2 / (2 ls_hi^2)) where
 // the query crosses its support, and 2N (cells crossed + 1) crossings per octave
-// are allowed for, as for single-octave media.  Returns the steps after the
-// evaluated point that keep the sign of f (margins as for single-octave media).
+// are allowed for, as for single-octave media.  Returns the steps on either side of
+// the evaluated point that keep the sign of f (margins as for single-octave media).
 //
 // The sums over the octaves factor into the local scale's terms and the flight's
 // constants of skip_consts (L.sk).  On the multi-resolution grid N = sum_j w_j (S_j /
@@ -3809,7 +3810,8 @@ __device__ __forceinline__ int oct_skip_count(const DevMedium &m, const LaneFiel
 // U |h| - D h + curv h^2 / 2 over a distance h, D the derivative of |f|: within the root of
 // that quadratic, and one cell's travel, every step has the sign of f.  A bound from the
 // slope alone (all 3 N splats at their steepest) reaches one step at |f| = 0.07 on the
-// sphere field where this one reaches four: 23.9 -> 13.7 evaluations per flight.
+// sphere field where this one reaches four: 12.7 evaluations per primary flight, 23.9 with
+// that bound on both sides.
 __device__ __forceinline__ void reach_1d(const LaneField &L, const float d[3], const float p[3], float f, int sg,
                                          float slope, float curv, float j0, float j1, float dn, float step, int cap,
                                          int &back, int &fore)
