@@ -2820,7 +2820,9 @@ struct LevelOrigin {
     float oz[2];
 };
 
-template <bool LEVELS = true>
+// LEVELS: the batch has multi-resolution media (with their code in its evaluators 60 013
+// three-octave flights took 3.84 ms a batch, without 3.43)
+template <bool LEVELS>
 __device__ __forceinline__ FastPoint fast_point(const LaneField &L, float px, float py, float pz, LevelOrigin &lo)
 {
     const DevMedium &m = *L.m;
@@ -2838,9 +2840,9 @@ __device__ __forceinline__ FastPoint fast_point(const LaneField &L, float px, fl
     if (q.mr) {
         q.ls = ls_value(m, px, pz);
         q.lv = mr_levels(m, q.ls);
-        if (L.cond) {
-            if (lo.s != q.lv.s[0]) {
-                lo.s = q.lv.s[0];
+        if (lo.s != q.lv.s[0]) {
+            lo.s = q.lv.s[0];
+            if (L.cond) {
 #pragma unroll
                 for (int j = 0; j < 2; ++j) lo.oz[j] = ray_coord_oct(m, L.n, L.o[0], L.o[1], L.o[2], q.lv.s[j]);
             }
@@ -2940,8 +2942,9 @@ constexpr uint32_t kHandOverPlain = 8, kHandOverGeneral = 4;
 // whose sums keep the cooperative evaluators' order and which takes the slope along; the
 // resume passes' values keep the one-lane evaluators' order, so that a miss has the same
 // bits whichever of them ends it.
-template <bool STAT, bool FAST>
+template <bool STAT, bool FAST, bool LEVELS = !STAT>
 struct EvalGroup1D {
+    static constexpr bool kLevels = LEVELS;
     static constexpr bool kCollective = false;
     static constexpr int kGroup = 8;
     static constexpr int kMinBlocks = 2;
@@ -3123,7 +3126,7 @@ struct EvalGroup1D {
             }
             return L.sigma * noise + lane_mean(L, px, py, pz, id);
         } else if constexpr (FAST) {
-            const FastPoint q = fast_point(L, px, py, pz, lo);
+            const FastPoint q = fast_point<LEVELS>(L, px, py, pz, lo);
             const int n_oct = q.mr ? 2 : (int)L.m->n_oct;
             last_ls = q.ls;
             float total = 0.0f;
@@ -3212,8 +3215,9 @@ struct EvalGroup1D {
 // 2 863 / 2 999, 80 000 4 186 / 4 127, 150 000 5 834 / 5 672, 300 007 10 229 / 9 489; a
 // nonstationary octave, 80 000 2 583 / 2 386; multi-resolution, 80 000 3 725 / 3 548.
 constexpr uint32_t kFewWarps = 12000, kFewWarpsPrecise = 60000;
-template <bool FAST>
+template <bool FAST, bool LEVELS = true>
 struct EvalWarp1D {
+    static constexpr bool kLevels = LEVELS;
     static constexpr bool kCollective = false;
     static constexpr int kGroup = 32;
     static constexpr int kMinBlocks = 2;
@@ -3257,7 +3261,7 @@ struct EvalWarp1D {
         uint32_t drawn = 0u;            // (the eights beyond the last octave repeat its cells)
         float vs, gz, oz;
         if constexpr (FAST) {
-            const FastPoint q = fast_point(L, px, py, pz, lo);
+            const FastPoint q = fast_point<LEVELS>(L, px, py, pz, lo);
             last_ls = q.ls;
             own(L, q.mr ? 0 : i, vs, gz, oz);
             const float z = fast_coord(L, q, i);
@@ -3605,8 +3609,8 @@ struct EvalCoop1D {
 // 1D evaluator for media with several octaves, a nonstationary length scale or the
 // multi-resolution grid (whose two levels count as octaves here): each octave's
 // three-cell impulse window lives in shared memory, and the cells of all octaves are drawn
-// together (window_fill).  NOCT: the most octaves (or levels) of the batch's media.  Every
-// lane of the warp must call value().
+// together (window_fill).  NOCT: the most octaves (or levels) of the batch's media, LEVELS: some
+// are on the grid.  Every lane of the warp must call value().
 //
 // What bounds it: issue slots and the instruction cache.  Drawing per octave and slot
 // (nine ballots and loops per evaluation), taking the skip bound's per-flight terms and
@@ -3614,8 +3618,9 @@ struct EvalCoop1D {
 // flight's set-up inside the march cost 2 540 instructions per lane and evaluation.
 constexpr int kOctMax = 4;
 
-template <int NOCT>
+template <int NOCT, bool LEVELS>
 struct EvalCoopOct {
+    static constexpr bool kLevels = LEVELS;
     static constexpr bool kCollective = true;
     static constexpr int kGroup = 1;
     static constexpr int kMinBlocks = 2;
@@ -3643,7 +3648,7 @@ struct EvalCoopOct {
     __device__ __forceinline__ float value(const LaneField &L, float px, float py, float pz,
                                            int &id, uint32_t &refills, bool live)
     {
-        const FastPoint q = fast_point<(NOCT > 1)>(L, px, py, pz, lo);
+        const FastPoint q = fast_point<LEVELS>(L, px, py, pz, lo);
         const int n_oct = live ? (q.mr ? 2 : (int)L.m->n_oct) : 0;
         last_ls = q.ls;
         if (q.mr && q.lv.seed[0] != level) {
@@ -3749,8 +3754,10 @@ constexpr int kMaxSkip3D = 32;
 // times the largest |S_j / norm + ow_j C_j|.  Where the span may leave the interval
 // between the two levels nothing is skipped (the origin's weights go with the level's
 // place, so the conditioning jumps there).
-__device__ __forceinline__ int oct_skip_count(const DevMedium &m, const LaneField &L, float ls_p, float f, float step,
-                                              int cap)
+// level: the lower level's scale at the point, which the fast evaluators keep (0: unknown).
+template <bool LEVELS = true>
+__device__ __forceinline__ int oct_skip_count(const DevMedium &m, const LaneField &L, float ls_p, float level, float f,
+                                              float step, int cap)
 {
     if (m.skip_mean_lip < 0.0f) return 0;
     const float n3 = 3.0f * (float)m.n_imp;
@@ -3758,13 +3765,16 @@ __device__ __forceinline__ int oct_skip_count(const DevMedium &m, const LaneFiel
     float lip = L.sk[0], j0, j1;
     const float dls = L.sk[1];
     const float reach = dls * ((float)cap * step) + 1e-6f;
-    if (m.flags & MF_MULTIRES) {
-        MrLevels lv;
-        mr_scales(m, ls_p, lv);
-        if (!(ls_p - reach > lv.s[0] * 1.00001f && ls_p + reach < lv.s[1] * 0.99999f)) return 0;
-        const float is = __fdividef(1.0f, lv.s[0]);
+    if (LEVELS && (m.flags & MF_MULTIRES)) {
+        if (level == 0.0f) {
+            MrLevels lv;
+            mr_scales(m, ls_p, lv);
+            level = lv.s[0];
+        }
+        if (!(ls_p - reach > level * 1.00001f && ls_p + reach < level * (2.5f * 0.99999f))) return 0;
+        const float is = __fdividef(1.0f, level);
         lip += 1.0771f * m.skip_noise_lip * is * L.sk[3] + 1.4143f * (0.42888194f * is * L.sk[4] + 0.5f * L.sk[5]) +
-               1.8858f * dls * is * (n3 * m.inv_norm1d * L.sk[2] + L.sk[6] + 0.42888194f * lv.s[1] * L.sk[7]);
+               1.8858f * dls * is * (n3 * m.inv_norm1d * L.sk[2] + L.sk[6] + 1.0723f * level * L.sk[7]);
         const float jn = m.skip_jump * 2.02f * (float)m.n_imp;
         j0 = 6.0f * jn * L.sk[2];
         j1 = jn * (step * __fdividef(1.41f * is * L.sk[3], m.kr_iso));
@@ -3865,9 +3875,9 @@ __device__ __forceinline__ float skip_scale(const DevMedium &m, float px, float 
 
 // the evaluators whose fast pass skips by oct_skip_count
 template <class E> struct IsOct { static constexpr bool value = false; };
-template <int NOCT> struct IsOct<EvalCoopOct<NOCT>> { static constexpr bool value = true; };
-template <> struct IsOct<EvalWarp1D<true>> { static constexpr bool value = true; };
-template <> struct IsOct<EvalGroup1D<false, true>> { static constexpr bool value = true; };
+template <int NOCT, bool LEVELS> struct IsOct<EvalCoopOct<NOCT, LEVELS>> { static constexpr bool value = true; };
+template <bool LEVELS> struct IsOct<EvalWarp1D<true, LEVELS>> { static constexpr bool value = true; };
+template <bool LEVELS> struct IsOct<EvalGroup1D<false, true, LEVELS>> { static constexpr bool value = true; };
 
 template <class E> struct IsSkip3D { static constexpr bool value = false; };
 template <> struct IsSkip3D<EvalSkip3D> { static constexpr bool value = true; };
@@ -4235,7 +4245,8 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
             if constexpr (IsOct<Eval>::value) {
                 // the bound takes the worst local scale of the span, so the span follows
                 // the last reach, before a proposed interval too
-                back = fore = oct_skip_count(*L.m, L, ev.last_ls, f, step, min(max(2 * reach + 2, 4), limit));
+                back = fore = oct_skip_count<Eval::kLevels>(*L.m, L, ev.last_ls, ev.lo.s, f, step,
+                                                           min(max(2 * reach + 2, 4), limit));
                 reach = fore;
                 next = (3 * fore) >> 2;
             }
@@ -4433,7 +4444,8 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                 }
                 if constexpr (IsOct<Eval>::value) {
                     // (a longer span loosens the bound, whatever a proposal says)
-                    if (!RESUME) skip = oct_skip_count(*L.m, L, ev.last_ls, f, step, early ? min(prop_cap, kMaxSkip) : kMaxSkip);
+                    if (!RESUME) skip = oct_skip_count<Eval::kLevels>(*L.m, L, ev.last_ls, ev.lo.s, f, step,
+                                                                       early ? min(prop_cap, kMaxSkip) : kMaxSkip);
                 }
                 if constexpr (RESUME) {
                     // a flight that marches on after a decision skips by the same slope bound
@@ -4441,7 +4453,7 @@ __device__ __forceinline__ void march_flights(const FlightArgs &a)
                     // crossing is then no longer the last one evaluated, so the refinement
                     // re-evaluates it
                     if (!kOwn3D && !Eval::kSkip && (L.m->flags & MF_ONE_D))
-                        skip = oct_skip_count(*L.m, L, skip_scale(*L.m, p[0], p[2]), f, step, kMaxSkip);
+                        skip = oct_skip_count(*L.m, L, skip_scale(*L.m, p[0], p[2]), 0.0f, f, step, kMaxSkip);
                     else if (G == 1 && use3)
                         skip = ev3.skips(f, step, kMaxSkip3D);
                     if (skip > 0) pf_precise = false;
@@ -5167,6 +5179,29 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
         b.run_hi = hi;
         if (a.n >= few) groups();
     };
+    // the fast passes of general media, with the levels' code or without
+    auto by_levels = [&](auto pass) {
+        if (a.any_mr) pass(std::true_type());
+        else pass(std::false_type());
+    };
+    auto warps = [&](auto levels) {
+        using Warp = EvalWarp1D<true, decltype(levels)::value>;
+        k_march<Warp, false><<<grid((const void *)k_march<Warp, false>, 0, true, 32), 256, 0, stream>>>(b);
+    };
+    auto groups = [&](auto levels) {
+        using Group = EvalGroup1D<false, true, decltype(levels)::value>;
+        k_march<Group, false><<<grid((const void *)k_march<Group, false>, 0, true, 8), 256, 0, stream>>>(b);
+    };
+    auto tail_warps = [&](auto levels) {
+        using Warp = EvalWarp1D<true, decltype(levels)::value>;
+        k_march<Warp, false, false, true>
+            <<<grid((const void *)k_march<Warp, false, false, true>, 0, true, 32), 256, 0, stream>>>(b);
+    };
+    auto tail_groups = [&](auto levels) {
+        using Group = EvalGroup1D<false, true, decltype(levels)::value>;
+        k_march<Group, false, false, true>
+            <<<grid((const void *)k_march<Group, false, false, true>, 0, true, 8), 256, 0, stream>>>(b);
+    };
     if (group1) {
         cudaError_t failed = cudaSuccess;
         sized(a.n_dev != nullptr, plain ? kFewPlain : kFewGeneral, [&] {
@@ -5174,13 +5209,7 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
                 const void *fn = (const void *)k_march<EvalGroup1D<true, true>, false>;
                 k_march<EvalGroup1D<true, true>, false><<<grid(fn, 0, true, 8), 256, 0, stream>>>(b);
             } else {
-                by_octaves(kFewWarps, [&] {
-                    const void *fn = (const void *)k_march<EvalWarp1D<true>, false>;
-                    k_march<EvalWarp1D<true>, false><<<grid(fn, 0, true, 32), 256, 0, stream>>>(b);
-                }, [&] {
-                    const void *fn = (const void *)k_march<EvalGroup1D<false, true>, false>;
-                    k_march<EvalGroup1D<false, true>, false><<<grid(fn, 0, true, 8), 256, 0, stream>>>(b);
-                }, a.n_dev != nullptr);
+                by_octaves(kFewWarps, [&] { by_levels(warps); }, [&] { by_levels(groups); }, a.n_dev != nullptr);
             }
         }, [&] {
             b.hand_over = plain ? (a.all_grid ? 0u : kHandOverPlain) : kHandOverGeneral;
@@ -5189,17 +5218,22 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
                 // single octave, two also for the grid's levels): 1 048 576 flights of one
                 // octave 7.40 ms a batch, with loops to four 9.04; of two 14.3 / 15.6, 60 000
                 // on the grid 3.50 / 3.61
-                auto octaves = [&](auto count) {
-                    using Oct = EvalCoopOct<decltype(count)::value>;
+                auto octaves = [&](auto count, auto levels) {
+                    using Oct = EvalCoopOct<decltype(count)::value, decltype(levels)::value>;
                     const void *fn = (const void *)k_march<Oct, false>;
                     const size_t smem = smem_window(std::max<uint32_t>(a.max_oct, a.any_mr ? 2u : 1u));
                     failed = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                   (int)smem_window(decltype(count)::value));
                     k_march<Oct, false><<<grid(fn, smem), 256, smem, stream>>>(b);
                 };
-                if (a.max_oct == 1u && !a.any_mr) octaves(std::integral_constant<int, 1>());
-                else if (a.max_oct <= 2u) octaves(std::integral_constant<int, 2>());
-                else octaves(std::integral_constant<int, kOctMax>());
+                const std::integral_constant<int, 1> one;
+                const std::integral_constant<int, 2> two;
+                const std::integral_constant<int, kOctMax> most;
+                if (a.any_mr && a.max_oct <= 2u) octaves(two, std::true_type());
+                else if (a.any_mr) octaves(most, std::true_type());
+                else if (a.max_oct == 1u) octaves(one, std::false_type());
+                else if (a.max_oct == 2u) octaves(two, std::false_type());
+                else octaves(most, std::false_type());
             } else if (a.all_grid) {
                 using Grid = EvalCoop1D<8, true, true>;
                 const void *fn = (const void *)k_march<Grid, false>;
@@ -5220,13 +5254,7 @@ cudaError_t launch_flights(const FlightArgs &a, int num_sms, cudaStream_t stream
                 const void *fn = (const void *)k_march<EvalGroup1D<true, true>, false, false, true>;
                 k_march<EvalGroup1D<true, true>, false, false, true><<<grid(fn, 0, true, 8), 256, 0, stream>>>(b);
             } else {
-                by_octaves(kFewWarps, [&] {
-                    const void *fn = (const void *)k_march<EvalWarp1D<true>, false, false, true>;
-                    k_march<EvalWarp1D<true>, false, false, true><<<grid(fn, 0, true, 32), 256, 0, stream>>>(b);
-                }, [&] {
-                    const void *fn = (const void *)k_march<EvalGroup1D<false, true>, false, false, true>;
-                    k_march<EvalGroup1D<false, true>, false, false, true><<<grid(fn, 0, true, 8), 256, 0, stream>>>(b);
-                }, true);
+                by_octaves(kFewWarps, [&] { by_levels(tail_warps); }, [&] { by_levels(tail_groups); }, true);
                 b.run_lo = 0;
                 b.run_hi = all;
             }
