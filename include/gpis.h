@@ -467,7 +467,9 @@ typedef struct {
 } gpis_render_stats;
 
 /* Render into image_rgb (host, height x width x 3 floats, row 0 at the top):
- * the mean radiance of spp paths per pixel.  Blocking.                       */
+ * the mean radiance of spp paths per pixel.  Blocking.  The context keeps its
+ * render buffers of up to 256 MiB until it is destroyed; larger ones are freed
+ * when the render returns.                                                   */
 int gpis_render(gpis_ctx *ctx, const gpis_scene_desc *scene, float *image_rgb, gpis_render_stats *stats);
 /* Render n_scenes scenes (each with its own medium of the context, image size,
  * spp and bounces) in one wavefront: their paths share every flight batch.
